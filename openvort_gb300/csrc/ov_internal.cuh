@@ -83,6 +83,8 @@ enum MemberWords {
 constexpr int TREE_LV_SLOTS = 32;   // levels 0..OV_MAX_LEVEL of the per-level cell lists
 constexpr int TREE_INV_COUNT = 4096; // table of 1 / count for the cell means
 
+struct CellFX;             // 64 bytes: fixed-point view for the FP64 path (ov_fxlaw.cuh)
+
 struct TreeBuf {
     int cap = 0;
     int *tt = nullptr;           // TT_WORDS ints per member
@@ -98,6 +100,7 @@ struct TreeBuf {
     Cell64 *cells = nullptr;
     Cell32 *cells32 = nullptr;
     CellFF *cellsff = nullptr;
+    CellFX *cellsfx = nullptr;
     double *psum = nullptr;      // 3 doubles per cell of more than one node: position sum (a one-node
                                  // cell's mean is its sum; every cell's circulation is a sum)
     uint8_t *lvl8 = nullptr;     // level of each cell (0 for roots)
@@ -357,6 +360,10 @@ int ov_upload_member_tables(ov_ctx *c);
 int ov_move_device_slots(ov_ctx *c, const std::vector<Member> &old);
 void ov_tree_free(TreeBuf &t);
 int ov_tree_build(ov_ctx *c, const NodeArrays &na, cudaStream_t s);
+// Unit of the integer law's coordinates: grid step / 2^bits, every separation
+// below 2^61 units (a box's grid leaves two periods of room, a spherical
+// section's none).
+inline int ov_fx_bits(const ov_ctx *c) { return c->geo.sph ? 38 : 39; }
 
 // sort / scan (ov_sort.cu)
 void ov_sort_keys(ov_ctx *c, TreeBuf &t, int n, cudaStream_t s);

@@ -23,6 +23,7 @@
 // is empty and the keys hold 21 levels; with T members it takes
 // ceil(log2 T) bits and the keys hold floor((63 - bits) / 3) levels.
 #include "ov_internal.cuh"
+#include "ov_fxlaw.cuh"
 
 void ov_sort_keys(ov_ctx *c, TreeBuf &t, int n, cudaStream_t s);
 int ov_sort_hist_ints(int cap);
@@ -446,11 +447,49 @@ __device__ __forceinline__ void write_cellff(CellFF *out, int ci, const double c
     out[ci] = o;
 }
 
+// Fixed-point view for the FP64 path's integer law (ov_fxlaw.cuh): centre of
+// mass and circulation in units 1 / fx_inv, the circulation left-normalised.
+__device__ __forceinline__ void write_cellfx(CellFX *out, int ci, const double c[3], const double q[3], double fx_inv)
+{
+    CellFX o;
+    uint64_t m = 0;
+    bool fits = true;
+    int64_t s[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const double x = c[a] * fx_inv, y = q[a] * fx_inv;
+        fits = fits && fabs(x) < 2305843009213693952.0 && fabs(y) < 2305843009213693952.0;   // 2^61
+        o.c[a] = __double2ll_rn(x);
+        s[a] = __double2ll_rn(y);
+        m |= (uint64_t)(s[a] < 0 ? -s[a] : s[a]);
+    }
+    o.e = fits ? (m ? __clzll((long long)m) - 3 : kFxZero) : kFxNone;
+    o.n = 0;
+    int64_t low = 0;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const fx_split p = fx_parts(o.e > 0 ? (int64_t)((uint64_t)s[a] << o.e) : s[a]);
+        o.sh[a] = p.h;
+        o.sl[a] = p.l;
+        o.n += fx_mul(p.h, p.h);
+        low += fx_mul(p.h, p.l);
+    }
+    o.n += low >> 31;
+    o.pad = 0;
+    const int4 *src = reinterpret_cast<const int4 *>(&o);
+    int4 *dst = reinterpret_cast<int4 *>(out + ci);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) dst[i] = src[i];
+}
+
 // What the traversals read of a cell once its sums are known: the means and
-// the circulation in the FP64 cell, the FP32 and double-single views.
+// the circulation in the FP64 cell, the FP32, double-single and fixed-point
+// views.
 struct CellViews {
     Cell32 *c32;
     CellFF *cff;
+    CellFX *cfx;
+    double fx_inv;
     double h, inv_h, theta;
     const double *inv_count;   // 1 / k for k < TREE_INV_COUNT
     const float *lev_tab;      // box cells: threshold and Lm per level (null: spherical cells)
@@ -481,6 +520,7 @@ __device__ __forceinline__ void store_cell(Cell64 *cells, int ci, const double s
         write_cell32(v.c32, ci, c, q, thr, lm32, next, v.h, v.inv_h);
     }
     if (v.cff) write_cellff(v.cff, ci, c, q, v.h, v.inv_h);
+    if (v.cfx) write_cellfx(v.cfx, ci, c, q, v.fx_inv);
 }
 
 __device__ __forceinline__ void store_psum(double *psum, int ci, const double acc[6])
@@ -852,6 +892,7 @@ __global__ void k_root(const int *__restrict__ order, const int *__restrict__ ce
         write_cell32(views.c32, root, c, q, cell_thr(r.lm, views.theta), __double2float_ru(r.lm), r.next, views.h,
                      views.inv_h);
     if (views.cff) write_cellff(views.cff, root, c, q, views.h, views.inv_h);
+    if (views.cfx) write_cellfx(views.cfx, root, c, q, views.fx_inv);
 }
 
 }  // namespace
@@ -860,16 +901,17 @@ int ov_tree_reserve_cells(ov_ctx *c, int cells)
 {
     TreeBuf &t = c->tree;
     if (t.cap_cells >= cells && t.cells) return OV_OK;
-    void *ptrs[] = {t.cells, t.cells32, t.cellsff, t.psum, t.first, t.lvl_list, t.lvl8};
+    void *ptrs[] = {t.cells, t.cells32, t.cellsff, t.cellsfx, t.psum, t.first, t.lvl_list, t.lvl8};
     for (void *p : ptrs)
         if (p) cudaFree(p);
-    t.cells = nullptr; t.cells32 = nullptr; t.cellsff = nullptr; t.first = t.lvl_list = nullptr;
+    t.cells = nullptr; t.cells32 = nullptr; t.cellsff = nullptr; t.cellsfx = nullptr; t.first = t.lvl_list = nullptr;
     t.psum = nullptr;
     t.lvl8 = nullptr;
     t.cap_cells = 0;
     OV_ALLOC(c, cudaMalloc(&t.cells, (size_t)cells * sizeof(Cell64)));
     OV_ALLOC(c, cudaMalloc(&t.cells32, (size_t)cells * sizeof(Cell32)));
     OV_ALLOC(c, cudaMalloc(&t.cellsff, (size_t)cells * sizeof(CellFF)));
+    OV_ALLOC(c, cudaMalloc(&t.cellsfx, (size_t)cells * sizeof(CellFX)));
     OV_ALLOC(c, cudaMalloc(&t.psum, (size_t)cells * 3 * 8));
     OV_ALLOC(c, cudaMalloc(&t.lvl8, (size_t)cells));
     OV_ALLOC(c, cudaMalloc(&t.first, (size_t)cells * 4));
@@ -917,7 +959,7 @@ int ov_tree_reserve(ov_ctx *c, int cap)
 void ov_tree_free(TreeBuf &t)
 {
     void *ptrs[] = {t.keys, t.keys_alt, t.order, t.order_alt, t.torder, t.cpl, t.ncell_at, t.cell_off, t.scan_tmp,
-                    t.sort_hist, t.cells, t.cells32, t.cellsff, t.psum, t.first, t.lvl_list, t.lvl8, t.lvl_cnt, t.nm, t.lev_tab, t.inv_count,
+                    t.sort_hist, t.cells, t.cells32, t.cellsff, t.cellsfx, t.psum, t.first, t.lvl_list, t.lvl8, t.lvl_cnt, t.nm, t.lev_tab, t.inv_count,
                     t.counters, t.tt};
     for (void *p : ptrs)
         if (p) cudaFree(p);
@@ -993,6 +1035,8 @@ int ov_tree_build(ov_ctx *c, const NodeArrays &na, cudaStream_t s)
     const bool fp32_view = c->precision == OV_PREC_MIXED || c->precision == OV_PREC_DD || c->walk == OV_WALK_SPLIT;
     views.c32 = fp32_view ? t.cells32 : nullptr;
     views.cff = c->precision == OV_PREC_DD ? t.cellsff : nullptr;
+    views.cfx = c->precision != OV_PREC_MIXED && c->walk == OV_WALK_SPLIT ? t.cellsfx : nullptr;
+    views.fx_inv = ldexp(1.0 / c->grid_h, ov_fx_bits(c));
     views.h = c->grid_h;
     views.inv_h = 1.0 / c->grid_h;
     views.theta = c->params.bh_resolution;

@@ -19,6 +19,7 @@
 #include <algorithm>
 
 #include "ov_internal.cuh"
+#include "ov_fxlaw.cuh"
 
 #ifndef M_PI
 #define M_PI 3.14159265358979323846
@@ -43,6 +44,8 @@ struct VelArgs {
     const Cell64 *cells;
     const Cell32 *cells32;
     const CellFF *cellsff;      // OV_PREC_DD: double-single cell data
+    const CellFX *cellsfx;      // FP64 split walk: fixed-point cell data
+    double fx_inv;              // 1 / its unit (a power of two)
     const double *x, *y, *z, *tx, *ty, *tz, *nx, *ny, *nz;
     double *vx, *vy, *vz, *sx, *sy, *sz;
     const int *fwd, *rev, *status, *pin;
@@ -284,19 +287,21 @@ __device__ __forceinline__ void image_point(const Geometry &g, int j, const doub
 #pragma unroll
     for (int ax = 0; ax < 3; ++ax) q[ax] = rn_sub(p[ax], rn_mul(g.L[ax], (double)g.shift[j][ax]));
     for (int m = 0; m < g.nreflect[j]; ++m) {
-        int f = g.reflect[j][m];
+        const int f = g.reflect[j][m];
         if (f < 0 || f > 5) continue;
-        int ax = f >> 1;
-        double w = (f & 1) ? g.hi[ax] : g.lo[ax];
-        q[ax] = rn_sub(rn_mul(2.0, w), p[ax]);
+        // (selected, not indexed: the arrays stay in registers)
+#pragma unroll
+        for (int ax = 0; ax < 3; ++ax)
+            if (f >> 1 == ax) q[ax] = rn_sub(rn_mul(2.0, (f & 1) ? g.hi[ax] : g.lo[ax]), p[ax]);
     }
 }
 
 __device__ __forceinline__ void mirror_vec(int f, double v[3])
 {
     // mirror_vector_reflect (boundaries.c:201-211): normal component flips
-    int ax = f >> 1;
-    v[ax] = -v[ax];
+#pragma unroll
+    for (int ax = 0; ax < 3; ++ax)
+        if (f >> 1 == ax) v[ax] = -v[ax];
 }
 
 // The segment law (octree.c:321-342 / tangle.c:536-559) for R = COM - r
@@ -1468,81 +1473,106 @@ __global__ void __launch_bounds__(32 * W, (min_blocks_mixp<W, R>())) k_vel_mixp(
 // The walk (distance and opening tests) runs in FP32 on the grid-split cells
 // exactly as the mixed traversal's, with the FP64 test inside the guard
 // bands, so every lane accepts, skips and opens the cells the FP64 walk
-// does.  Accepted cells go to the lane's list in shared memory.  When a list
-// nears its capacity, and at the end of each query point, the warp
-// evaluates all lists together in FP64, 32 entries at a time whoever owns
-// them (the owner's query point comes by shuffle), and every owner adds its
-// own terms in walk order (the FP64 walk's summation order).  GB300 runs
-// FP64 at 1/64 of the FP32 rate: this keeps the FP64 pipe for the
-// interactions, in warp instructions with all lanes busy, instead of
-// spending it on every visited cell and on idle lanes.
+// does.  Accepted cells go to the lane's list in shared memory; each lane
+// then evaluates its own list with the integer-mantissa law (ov_fxlaw.cuh),
+// which leaves the FP64 pipe (1/64 of the FP32 rate) one conversion and one
+// multiply-add per component.  Evaluating in the walk would leave 43 % of
+// the lanes idle in the law; neighbouring targets' lists are alike, so own
+// lists keep 85 % of them busy without redistributing entries.
 
-constexpr int kListCap = 64;   // accepted cells per lane between evaluations
+constexpr int kListCap = 48;    // accepted cells per lane between evaluations
+constexpr int kListStep = 8;    // walk steps between tests of the lists' lengths
+constexpr int kLateCap = 8;     // of them, cells left to the FP64 law per query point
 
-// A warp's lists and the scratch of their evaluation (shared memory).
+// A warp's lists, and per lane what the walks need rarely: the query point in
+// FP64 and the node's position split on the grid.
 struct WarpLists {
     int entry[kListCap * 32];   // entry i of lane l at [32 i + l]
-    unsigned row_mask[kListCap];   // row i: the lanes holding an entry i
-    int row_start[kListCap];       // entries in rows before row i
-    double w[32][3];               // the terms of one batch of 32 entries
+    int late[kLateCap * 32];
+    int nlate[32];
+    double q[3][32];
+    float g0[3][32], f0[3][32];
 };
+extern __shared__ WarpLists s_lists[];   // one per warp of the block
 
-// Evaluate the warp's lists (this lane holds n entries) at the lanes' query
-// points q and add each lane's terms to its v, in entry order.
-__device__ __forceinline__ void flush_lists(const VelArgs &a, WarpLists &L, int lane, int n, const double q[3],
-                                            double v[3])
+__device__ __forceinline__ CellFX load_cellfx(const CellFX *p)
 {
-    const int nmax = __reduce_max_sync(0xffffffffu, n);
-    if (nmax == 0) return;
-    // rows, in entry order: row i holds the i-th entry of every lane that has one
-    int total = 0;
-    for (int i = 0; i < nmax; ++i) {
-        const unsigned m = __ballot_sync(0xffffffffu, n > i);
-        if (lane == 0) { L.row_mask[i] = m; L.row_start[i] = total; }
-        total += __popc(m);
-    }
-    __syncwarp();
-    const unsigned below = (1u << lane) - 1u;
-    int own = 0;   // this lane's next entry to add
-    for (int base = 0; base < total; base += 32) {
-        // entry base + lane: its row (the last one starting at or before it) and owner
-        const int k = base + lane;
-        int owner = lane, cell = -1;
-        if (k < total) {
-            int lo = 0, hi = nmax - 1;
-            while (lo < hi) {
-                const int mid = (lo + hi + 1) >> 1;
-                if (L.row_start[mid] <= k) lo = mid; else hi = mid - 1;
-            }
-            owner = __fns(L.row_mask[lo], 0, k - L.row_start[lo] + 1);
-            cell = L.entry[32 * lo + owner];
-        }
-        double qo[3];
+    const int4 *src = reinterpret_cast<const int4 *>(p);
+    CellFX c;
+    int4 *dst = reinterpret_cast<int4 *>(&c);
 #pragma unroll
-        for (int ax = 0; ax < 3; ++ax) qo[ax] = __shfl_sync(0xffffffffu, q[ax], owner);
-        double w[3] = {0.0, 0.0, 0.0};
-        if (cell >= 0) law64_term(a.cells + cell, qo, w);
-        L.w[lane][0] = w[0]; L.w[lane][1] = w[1]; L.w[lane][2] = w[2];
-        __syncwarp();
-        // this lane's own entries in the batch, in order
-        while (own < n) {
-            const int ko = L.row_start[own] + __popc(L.row_mask[own] & below) - base;
-            if (ko >= 32) break;
-            v[0] += L.w[ko][0]; v[1] += L.w[ko][1]; v[2] += L.w[ko][2];
-            ++own;
-        }
-        __syncwarp();
-    }
+    for (int i = 0; i < 4; ++i) dst[i] = __ldg(src + i);
+    return c;
 }
 
-// One query point (split g + f for the tests, q in FP64 for the law) for the
-// 32 lanes of a warp; the lane's FP64 velocity in v.
+// Evaluate the last min(n, rows) entries of every lane's list at its query
+// point; the sum in units kappa / 4 pi / u.  Cells left to the FP64 law go to
+// the late list (or are evaluated when it is full).
+__device__ __forceinline__ double3 run_list(const CellFX *cells, const Cell64 *cells64, int rows, int n, double fx_inv)
+{
+    const int lane = threadIdx.x & 31;
+    WarpLists &L = s_lists[threadIdx.x >> 5];
+    int64_t q[3];
+    bool in_range = true;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const double x = L.q[i][lane] * fx_inv;
+        in_range = in_range && fabs(x) < 2305843009213693952.0;   // 2^61
+        q[i] = __double2ll_rn(x);
+    }
+    double v[3] = {0.0, 0.0, 0.0};
+    const double unit = ldexp(1.0, kFxUnit);
+    while (rows > 0) {
+        fx_sum sum[3] = {{0, 0}, {0, 0}, {0, 0}};
+        const int some = min(rows, kFxTerms);
+#pragma unroll 1
+        for (int k = 0; k < some; ++k) {
+            if (n == 0) continue;
+            const int cell = L.entry[32 * --n + lane];
+            const CellFX c = load_cellfx(cells + cell);
+            if (!fx_law(c, q, in_range, sum) && !(in_range && c.e == kFxZero)) {
+                const int late = L.nlate[lane];
+                if (late < kLateCap) {
+                    L.late[32 * late + lane] = cell;
+                    L.nlate[lane] = late + 1;
+                } else {
+                    const double qd[3] = {L.q[0][lane], L.q[1][lane], L.q[2][lane]};
+                    double w[3];
+                    law64_term(cells64 + cell, qd, w);
+                    for (int i = 0; i < 3; ++i) v[i] += w[i] / fx_inv;
+                }
+            }
+        }
+        rows -= some;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) v[i] = fma(fx_value(sum[i]), unit, v[i]);
+    }
+    return make_double3(v[0], v[1], v[2]);
+}
+
+// The cells left to the FP64 law, all lanes together.
+__device__ __noinline__ double3 run_late(const Cell64 *cells64, int rows)
+{
+    const int lane = threadIdx.x & 31;
+    WarpLists &L = s_lists[threadIdx.x >> 5];
+    const double q[3] = {L.q[0][lane], L.q[1][lane], L.q[2][lane]};
+    double v[3] = {0.0, 0.0, 0.0};
+    for (int k = 0; k < rows; ++k) {
+        if (k >= L.nlate[lane]) continue;
+        double w[3];
+        law64_term(cells64 + L.late[32 * k + lane], q, w);
+        for (int i = 0; i < 3; ++i) v[i] += w[i];
+    }
+    L.nlate[lane] = 0;
+    return make_double3(v[0], v[1], v[2]);
+}
+
 // The split walk's decision for cell c (A, B its first 32 bytes, nxt its
 // successor): the mixed traversal's FP32 tests outside their guard bands,
 // the FP64 path's (decide64) inside them.  0 open, 1 skip, 2 accept.
 __device__ __forceinline__ int split_decision(const VelArgs &a, int c, const float4 &A, const float4 &B, int nxt,
                                               const float g[3], const float f[3], const float2 &ng01,
-                                              const float2 &nf01, const double q[3], MixedAcc &m)
+                                              const float2 &nf01, const WarpLists &L, int lane, unsigned &nfb)
 {
     const float d2lo = 1e-16f * (1.0f - 1e-5f), d2hi = 1e-16f * (1.0f + 1e-5f);
     // x and y two-wide as (A - g) + (B - f) (ng01, nf01: -g and -f of x, y),
@@ -1556,8 +1586,9 @@ __device__ __forceinline__ int split_decision(const VelArgs &a, int c, const flo
     bool acc = !skip && (leaf || d2 > A.w);
     const bool opn = !skip && !leaf && d2 < A.w * kThrLo;
     if ((!skip && d2 <= d2hi) || (!skip && !acc && !opn)) {
-        ++m.nfb;
+        ++nfb;
         double dxyz[3], d64;
+        const double q[3] = {L.q[0][lane], L.q[1][lane], L.q[2][lane]};
         const int dec = decide64(a, a.cells + c, q, a.prm.theta, leaf, dxyz, &d64);
         skip = dec == 1;
         acc = dec == 2;
@@ -1572,9 +1603,9 @@ __device__ __forceinline__ int split_decision(const VelArgs &a, int c, const flo
 // from b on.  The decisions are the walk's own (split_decision); nothing is
 // counted.
 __device__ __forceinline__ int ancestor_resume(const VelArgs &a, int root, int end, int b, const float g[3],
-                                               const float f[3], const double q[3])
+                                               const float f[3], const WarpLists &L, int lane)
 {
-    MixedAcc tmp = {0, 0, 0, 0, 0, 0, 0u, 0u, 0u, 0u, 0u};
+    unsigned tmp = 0;
     const float2 ng01 = make_float2(-g[0], -g[1]), nf01 = make_float2(-f[0], -f[1]);
     int c = root;
     for (int guard = 0; c < b && guard < 32 * (OV_MAX_LEVEL + 2); ++guard) {
@@ -1582,7 +1613,7 @@ __device__ __forceinline__ int ancestor_resume(const VelArgs &a, int root, int e
         const float4 A = __ldg(cp4), B = __ldg(cp4 + 1);
         int nxt = __float_as_int(B.w);
         if (nxt <= c || nxt > end) { bad_index(a, 2, c); return 0x7fffffff; }
-        if (split_decision(a, c, A, B, nxt, g, f, ng01, nf01, q, tmp) != 0) return nxt;   // accepted or skipped
+        if (split_decision(a, c, A, B, nxt, g, f, ng01, nf01, L, lane, tmp) != 0) return nxt;   // accepted or skipped
         // opened: on to the child holding b
         int ch = c + 1;
         for (int k = 0; k < 8; ++k) {
@@ -1596,14 +1627,22 @@ __device__ __forceinline__ int ancestor_resume(const VelArgs &a, int root, int e
     return 0;
 }
 
+// Cells visited, accepted, decided in FP64 by a lane, and its warp's steps.
+struct WalkCounts {
+    unsigned nvis, nacc, nfb, nstep;
+};
+
+// One query point (split g + f for the tests, in FP64 in L.q) for the 32
+// lanes of a warp; the lane's velocity in v.
 // The walk of cells [root, ncell) stops at `stop` (a sub-walk's end; ncell
 // otherwise); successors are checked against ncell.  resume0: the lane takes
 // part from that cell on (0: from the start; INT_MAX: not at all).
-__device__ __forceinline__ void walk_split(const VelArgs &a, const float g[3], const float f[3], const double q[3],
-                                           int resume0, int root, int ncell, int stop, WarpLists &L, int lane,
-                                           double v[3], MixedAcc &m, bool &overflow)
+__device__ __forceinline__ void walk_split(const VelArgs &a, const float g[3], const float f[3], int resume0, int root,
+                                           int ncell, int stop, WarpLists &L, int lane, double v[3], WalkCounts &m,
+                                           bool &overflow)
 {
-    v[0] = v[1] = v[2] = 0;
+    v[0] = v[1] = v[2] = 0.0;
+    L.nlate[lane] = 0;
     const float2 ng01 = make_float2(-g[0], -g[1]), nf01 = make_float2(-f[0], -f[1]);
     int c = root;
     int resume = resume0;
@@ -1619,7 +1658,7 @@ __device__ __forceinline__ void walk_split(const VelArgs &a, const float g[3], c
         bool open = false;
         if (c >= resume) {
             ++m.nvis;
-            const int dec = split_decision(a, c, A, B, nxt, g, f, ng01, nf01, q, m);
+            const int dec = split_decision(a, c, A, B, nxt, g, f, ng01, nf01, L, lane, m.nfb);
             if (dec == 2) {
                 ++m.nacc;
                 L.entry[32 * n + lane] = c;
@@ -1632,21 +1671,34 @@ __device__ __forceinline__ void walk_split(const VelArgs &a, const float g[3], c
             }
         }
         ++steps;
-        // a lane adds at most one entry a step: room for 16 more after this test
-        if ((steps & 15) == 0 && __any_sync(0xffffffffu, n > kListCap - 16)) {
-            flush_lists(a, L, lane, n, q, v);
-            n = 0;
+        // a lane adds at most one entry a step: room for kListStep more after this test
+        if ((steps & (kListStep - 1)) == 0 && __any_sync(0xffffffffu, n > kListCap - kListStep)) {
+            const double3 w = run_list(a.cellsfx, a.cells, kListCap / 2, n, a.fx_inv);
+            n = max(n - kListCap / 2, 0);
+            v[0] += w.x; v[1] += w.y; v[2] += w.z;
         }
         c = __any_sync(0xffffffffu, open) ? c + 1 : nxt;
         if (steps > guard_max) { overflow = true; break; }
     }
-    flush_lists(a, L, lane, n, q, v);
-    v[0] *= a.f4pi; v[1] *= a.f4pi; v[2] *= a.f4pi;
+    const double scale = a.f4pi * a.fx_inv;   // (a power of two: the same rounding)
+    {
+        const double3 w = run_list(a.cellsfx, a.cells, __reduce_max_sync(0xffffffffu, n), n, a.fx_inv);
+        v[0] = (v[0] + w.x) * scale; v[1] = (v[1] + w.y) * scale; v[2] = (v[2] + w.z) * scale;
+    }
+    const int late = __reduce_max_sync(0xffffffffu, L.nlate[lane]);
+    if (late > 0) {
+        const double3 w = run_late(a.cells, late);
+        v[0] = fma(w.x, a.f4pi, v[0]); v[1] = fma(w.y, a.f4pi, v[1]); v[2] = fma(w.z, a.f4pi, v[2]);
+    }
     m.nstep += steps;
 }
 
-// Resident blocks per SM the register budget is sized for (about 20 warps)
-template <int W> constexpr int min_blocks_split() { return W == 2 ? 10 : (W == 4 ? 5 : 2); }
+// Resident blocks per SM the register budget is sized for: 16 warps.  The law
+// runs at the integer pipe's rate from 8 warps on (cycles per 32 entries and
+// scheduler: 710 with 2 warps, 633 with 4, 602 with 8), and more lists leave
+// less L1 for the cells (65,536 nodes: 3.71 ms with 16 warps, 3.77 with 20,
+// 4.5 with 24).
+template <int W> constexpr int min_blocks_split() { return W == 2 ? 8 : (W == 4 ? 4 : 2); }
 
 template <int W>
 __global__ void __launch_bounds__(32 * W, min_blocks_split<W>()) k_vel_split(VelArgs a, double *__restrict__ part_out)
@@ -1654,9 +1706,8 @@ __global__ void __launch_bounds__(32 * W, min_blocks_split<W>()) k_vel_split(Vel
     const int lane = threadIdx.x & 31;
     const int tiles = a.counters[TC_ITEMS];
     const int items = tiles * a.G * a.S;
-    __shared__ WarpLists s_lists[W];
     WarpLists &lists = s_lists[threadIdx.x >> 5];
-    unsigned long long visits = 0, accepts = 0, steps = 0, fallback = 0;
+    unsigned visits = 0, accepts = 0, steps = 0, fallback = 0;   // per lane
     bool overflow = false;
     for (int it = next_item(a); it < items; it = next_item(a)) {
         const WorkItem w = decode_item(a, it, tiles);
@@ -1667,39 +1718,43 @@ __global__ void __launch_bounds__(32 * W, min_blocks_split<W>()) k_vel_split(Vel
         if (valid && (id < 0 || id >= a.cap)) { bad_index(a, 4, id); valid = false; id = 0; }
         const int st = valid ? a.status[id] : OV_EMPTY;
         const bool part = valid && st != OV_PINNED && st != OV_EMPTY && a.prm.use_bh;
-        double p[3] = {0, 0, 0};
-        if (valid) { p[0] = a.x[id]; p[1] = a.y[id]; p[2] = a.z[id]; }
-        float g0[3], f0[3];
+        {
+            const double p[3] = {valid ? a.x[id] : 0.0, valid ? a.y[id] : 0.0, valid ? a.z[id] : 0.0};
 #pragma unroll
-        for (int ax = 0; ax < 3; ++ax) {
-            const double G = rint(p[ax] * a.inv_h) * a.grid_h;
-            g0[ax] = (float)G;
-            f0[ax] = (float)(p[ax] - G);
+            for (int ax = 0; ax < 3; ++ax) {
+                const double G = rint(p[ax] * a.inv_h) * a.grid_h;
+                lists.g0[ax][lane] = (float)G;
+                lists.f0[ax][lane] = (float)(p[ax] - G);
+            }
         }
-        MixedAcc m = {0, 0, 0, 0, 0, 0, 0u, 0u, 0u, 0u, 0u};
-        double prim[3] = {0, 0, 0}, img[3] = {0, 0, 0};
+        WalkCounts m = {0u, 0u, 0u, 0u};
+        double *out = part_out + ((2 * ((size_t)w.grp * a.S + w.sub)) * 3) * (size_t)a.cap + tix;
+        double img[3] = {0, 0, 0};
+        bool own = false;   // the group holds the node's own point
         for (int qi = w.grp; qi <= a.geo.n_img; qi += a.G) {
             const int j = qi - 1;
-            double q[3];
+            {
+                double q[3] = {0.0, 0.0, 0.0};
+                if (valid) {
+                    const double p[3] = {a.x[id], a.y[id], a.z[id]};
+                    if (j < 0) { q[0] = p[0]; q[1] = p[1]; q[2] = p[2]; }
+                    else image_point(a.geo, j, p, q);
+                }
+                for (int ax = 0; ax < 3; ++ax) lists.q[ax][lane] = q[ax];
+            }
             float g[3], f[3];
-            if (j < 0) {
-                q[0] = p[0]; q[1] = p[1]; q[2] = p[2];
-                for (int ax = 0; ax < 3; ++ax) { g[ax] = g0[ax]; f[ax] = f0[ax]; }
+            if (j >= 0 && a.geo.nreflect[j] > 0) {
+                // a mirror image: the reflected point split on the grid
+                for (int ax = 0; ax < 3; ++ax) {
+                    const double q = lists.q[ax][lane], G = rint(q * a.inv_h) * a.grid_h;
+                    g[ax] = (float)G;
+                    f[ax] = (float)(q - G);
+                }
             } else {
-                image_point(a.geo, j, p, q);
-                if (a.geo.nreflect[j] > 0) {
-                    // a mirror image: the reflected point split on the grid
-                    for (int ax = 0; ax < 3; ++ax) {
-                        const double G = rint(q[ax] * a.inv_h) * a.grid_h;
-                        g[ax] = (float)G;
-                        f[ax] = (float)(q[ax] - G);
-                    }
-                } else {
-                    // p - L*shift: grid parts subtract exactly
-                    for (int ax = 0; ax < 3; ++ax) {
-                        g[ax] = g0[ax] - a.shift_g[j][ax];
-                        f[ax] = f0[ax] - a.shift_f[j][ax];
-                    }
+                // p - L*shift: grid parts subtract exactly
+                for (int ax = 0; ax < 3; ++ax) {
+                    g[ax] = lists.g0[ax][lane] - (j < 0 ? 0.0f : a.shift_g[j][ax]);
+                    f[ax] = lists.f0[ax][lane] - (j < 0 ? 0.0f : a.shift_f[j][ax]);
                 }
             }
             double v[3];
@@ -1711,23 +1766,23 @@ __global__ void __launch_bounds__(32 * W, min_blocks_split<W>()) k_vel_split(Vel
                 const long long nc = (long long)(w.end - w.root);
                 c0 = w.root + (int)(nc * w.sub / a.S);
                 c1 = w.root + (int)(nc * (w.sub + 1) / a.S);
-                if (part && c0 > w.root && c0 < c1) resume0 = ancestor_resume(a, w.root, w.end, c0, g, f, q);
+                if (part && c0 > w.root && c0 < c1) resume0 = ancestor_resume(a, w.root, w.end, c0, g, f, lists, lane);
             }
-            walk_split(a, g, f, q, resume0, c0, w.end, c1, lists, lane, v, m, overflow);
+            walk_split(a, g, f, resume0, c0, w.end, c1, lists, lane, v, m, overflow);
             if (j < 0) {
-                prim[0] = v[0]; prim[1] = v[1]; prim[2] = v[2];
+                own = true;
+                if (valid)
+                    for (int ax = 0; ax < 3; ++ax) out[(size_t)ax * a.cap] = v[ax];
             } else {
                 for (int r = 0; r < a.geo.nreflect[j]; ++r) mirror_vec(a.geo.reflect[j][r], v);
                 img[0] = rn_add(img[0], v[0]); img[1] = rn_add(img[1], v[1]); img[2] = rn_add(img[2], v[2]);
             }
         }
-        if (valid) {
-            const size_t cap = (size_t)a.cap, gs = (size_t)w.grp * a.S + w.sub;
+        if (valid)
             for (int ax = 0; ax < 3; ++ax) {
-                part_out[((2 * gs) * 3 + ax) * cap + tix] = prim[ax];
-                part_out[((2 * gs + 1) * 3 + ax) * cap + tix] = img[ax];
+                if (!own) out[(size_t)ax * a.cap] = 0.0;
+                out[(size_t)(3 + ax) * a.cap] = img[ax];
             }
-        }
         count_node(a, valid, id, m.nvis, m.nacc);
         visits += m.nvis;
         accepts += m.nacc;
@@ -1735,18 +1790,19 @@ __global__ void __launch_bounds__(32 * W, min_blocks_split<W>()) k_vel_split(Vel
         fallback += m.nfb;
     }
     int err = overflow ? OV_EW_ITER : 0;
+    unsigned long long v64 = visits, a64 = accepts, f64 = fallback;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-        visits += __shfl_xor_sync(0xffffffffu, visits, o);
-        accepts += __shfl_xor_sync(0xffffffffu, accepts, o);
-        fallback += __shfl_xor_sync(0xffffffffu, fallback, o);
+        v64 += __shfl_xor_sync(0xffffffffu, v64, o);
+        a64 += __shfl_xor_sync(0xffffffffu, a64, o);
+        f64 += __shfl_xor_sync(0xffffffffu, f64, o);
         err |= __shfl_xor_sync(0xffffffffu, err, o);
     }
     if (lane == 0) {
-        atomicAdd(&a.stat[ST_VISITS], visits);
-        atomicAdd(&a.stat[ST_ACCEPTS], accepts);
-        atomicAdd(&a.stat[ST_STEPS], steps);
-        atomicAdd(&a.stat[ST_FALLBACK], fallback);
+        atomicAdd(&a.stat[ST_VISITS], v64);
+        atomicAdd(&a.stat[ST_ACCEPTS], a64);
+        atomicAdd(&a.stat[ST_STEPS], (unsigned long long)steps);
+        atomicAdd(&a.stat[ST_FALLBACK], f64);
         if (err) atomicOr((int *)&a.counters[TC_ERR], err);
     }
 }
@@ -1754,15 +1810,16 @@ __global__ void __launch_bounds__(32 * W, min_blocks_split<W>()) k_vel_split(Vel
 }  // namespace
 
 // Query groups per node: the tuned value, else enough warps for ~32 per SM
-// on small tangles (~96 for the FP64 split walk, whose work items are
-// longer: finer items balance the end of the launch).
+// on small tangles (~400 for the FP64 split walk, whose work items are
+// longer: finer items balance the end of the launch.  65,536 nodes: 4.1 ms
+// with 8 groups, 3.9 with 14, 3.7 with 27).
 int ov_query_groups(ov_ctx *c)
 {
     int maxg = c->geo.n_img + 1;
     if (c->tune.groups > 0) return std::min(c->tune.groups, std::min(maxg, 27));
     int warps = (c->cap + 31) / 32;
     const bool split = c->precision == OV_PREC_FP64 && c->walk == OV_WALK_SPLIT;
-    const int per_sm = split ? 96 : 32, gmax = split ? 9 : 8;
+    const int per_sm = split ? 400 : 32, gmax = split ? 27 : 8;
     int G = (per_sm * c->sm_count + warps - 1) / warps;
     G = G < 1 ? 1 : (G > gmax ? gmax : G);
     return std::min(G, maxg);
@@ -1778,6 +1835,8 @@ VelArgs make_args(ov_ctx *c, const NodeArrays &na, double t, unsigned long long 
     a.cells = c->tree.cells;
     a.cells32 = c->tree.cells32;
     a.cellsff = c->tree.cellsff;
+    a.cellsfx = c->tree.cellsfx;
+    a.fx_inv = c->grid_h > 0 ? ldexp(1.0 / c->grid_h, ov_fx_bits(c)) : 0;
     a.x = na.x; a.y = na.y; a.z = na.z;
     a.tx = na.tx; a.ty = na.ty; a.tz = na.tz;
     a.nx = na.nx; a.ny = na.ny; a.nz = na.nz;
@@ -1914,13 +1973,24 @@ static VelKernel vel_kernel(int precision, int walk, int warps, int hi_occ, bool
     return k_vel_fp64<4>;
 }
 
+// Shared memory of the split walk's lists (0 for the other traversals); a
+// block of 8 warps needs the opt-in above 48 KB.
+static size_t list_bytes(const ov_ctx *c, int precision, int warps)
+{
+    if (precision != OV_PREC_FP64 || c->walk != OV_WALK_SPLIT) return 0;
+    if (warps == 8)
+        cudaFuncSetAttribute(k_vel_split<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * (int)sizeof(WarpLists));
+    return warps * sizeof(WarpLists);
+}
+
 // Persistent grid: resident blocks per SM (tuned or the occupancy limit) on
 // every SM, but no more blocks than there can be work items.
 int ov_traversal_blocks(ov_ctx *c, int precision, int warps, int *per_sm)
 {
     VelKernel k = vel_kernel(precision, c->walk, warps, c->tune.hi_occ, has_mirror_images(c->geo));
     int occ = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, 32 * warps, 0) != cudaSuccess || occ < 1) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, 32 * warps, list_bytes(c, precision, warps)) !=
+            cudaSuccess || occ < 1) {
         cudaGetLastError();
         occ = 1;
     }
@@ -1959,8 +2029,8 @@ int ov_launch_velocities(ov_ctx *c, const NodeArrays &na, double t, int precisio
         a.node_counts = c->d_node_counts;
     }
     OV_CUDA(c, cudaMemsetAsync(a.work, 0, sizeof(int), s));
-    vel_kernel(precision, c->walk, warps, c->tune.hi_occ, has_mirror_images(c->geo))<<<blocks, 32 * warps, 0, s>>>(
-        a, c->part);
+    vel_kernel(precision, c->walk, warps, c->tune.hi_occ, has_mirror_images(c->geo))<<<
+        blocks, 32 * warps, list_bytes(c, precision, warps), s>>>(a, c->part);
     if (a.S > 1) {
         const long long threads = 6LL * c->cap * a.G;
         k_part_sum<<<(unsigned)((threads + 127) / 128), 128, 0, s>>>(a, c->part);
@@ -3255,7 +3325,6 @@ __global__ void __launch_bounds__(128) k_sph_query_mixed(SphArgs s, double *__re
 __global__ void __launch_bounds__(128) k_sph_query_split(SphArgs s, double *__restrict__ part)
 {
     const VelArgs &a = s.v;
-    __shared__ WarpLists s_lists[4];
     const int lane = threadIdx.x & 31;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     WarpLists &lists = s_lists[threadIdx.x >> 5];
@@ -3288,10 +3357,11 @@ __global__ void __launch_bounds__(128) k_sph_query_split(SphArgs s, double *__re
         g[ax] = (float)G;
         f[ax] = (float)(qp[ax] - G);
     }
-    MixedAcc acc = {0, 0, 0, 0, 0, 0, 0u, 0u, 0u, 0u, 0u};
+    WalkCounts acc = {0u, 0u, 0u, 0u};
     bool overflow = false;
     double v[3];
-    walk_split(a, g, f, qp, go ? 0 : 0x7fffffff, root, end, end, lists, lane, v, acc, overflow);
+    for (int ax = 0; ax < 3; ++ax) lists.q[ax][lane] = qp[ax];
+    walk_split(a, g, f, go ? 0 : 0x7fffffff, root, end, end, lists, lane, v, acc, overflow);
     double w[3] = {v[0], v[1], v[2]};
     if (j >= 0) sph_rotate(v, -da, -dp, w);
     if (a.stat) {
@@ -3444,7 +3514,7 @@ int ov_launch_sph_velocities(ov_ctx *c, const SphDomain &d, const SphSettings &p
     if (c->precision == OV_PREC_MIXED)
         k_sph_query_mixed<<<(unsigned)((warps + 3) / 4), 128, 0, c->stream>>>(s, c->part);
     else if (c->walk == OV_WALK_SPLIT)
-        k_sph_query_split<<<(unsigned)((warps + 3) / 4), 128, 0, c->stream>>>(s, c->part);
+        k_sph_query_split<<<(unsigned)((warps + 3) / 4), 128, 4 * sizeof(WarpLists), c->stream>>>(s, c->part);
     else
         k_sph_query<<<(unsigned)((warps + 3) / 4), 128, 0, c->stream>>>(s, c->part);
     k_sph_finish<<<(d.n + 127) / 128, 128, 0, c->stream>>>(s, c->part);
