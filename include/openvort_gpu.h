@@ -91,9 +91,9 @@ enum {
                            (reference semantics; walk arithmetic: ov_set_walk) */
     OV_PREC_MIXED = 1,  /* FP32 traversal on grid-split positions, compensated sums,
                            FP64 for LIA, near field, guard-band decisions, RK4 update */
-    OV_PREC_DD = 2      /* the mixed traversal's FP32 walk and decisions, each accepted
-                           interaction and the sums in double-single (two floats, about
-                           1e-14 per operation): FP64-class accuracy at FP32 speed */
+    OV_PREC_DD = 2      /* FP64-class accuracy without the FP64 pipe: the mixed traversal's
+                           FP32 walk and decisions, each accepted interaction and the sums
+                           on 64-bit integer mantissas (the FP64 path's split walk) */
 };
 
 /* Download field mask for ov_download_tangle. */
@@ -141,7 +141,8 @@ int ov_set_precision(ov_ctx *ctx, int precision);
 enum {
     OV_WALK_SPLIT = 0,  /* default: the distance and opening tests in FP32 on
                            grid-split positions, the FP64 test inside their guard
-                           bands; accepted cells evaluated in FP64 by full warps */
+                           bands; accepted cells evaluated on 64-bit integer
+                           mantissas (at least FP64's accuracy), the nearest in FP64 */
     OV_WALK_FP64 = 1    /* every test in FP64 with the reference's rounding, each
                            accepted cell evaluated where the walk meets it */
 };

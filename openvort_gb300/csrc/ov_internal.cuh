@@ -62,13 +62,6 @@ struct Cell32 {          // 48 bytes: FP32 view for the FP32 walks; a walk step 
     float lm;            // Lm (rounded up)
 };
 
-struct CellFF {           // 64 bytes: double-single view for OV_PREC_DD
-    float g[3];          // centre of mass, grid part (exact, as in Cell32)
-    float fh[3], fl[3];  // centre of mass, the rest as hi + lo
-    float qh[3], ql[3];  // circulation, hi + lo
-    float pad;
-};
-
 // Per-member results of a forest build (tree.tt, TT_WORDS ints a member).
 enum MemberWords {
     TT_NNE = 0,   // non-EMPTY nodes
@@ -99,7 +92,6 @@ struct TreeBuf {
     int cap_cells = 0;
     Cell64 *cells = nullptr;
     Cell32 *cells32 = nullptr;
-    CellFF *cellsff = nullptr;
     CellFX *cellsfx = nullptr;
     double *psum = nullptr;      // 3 doubles per cell of more than one node: position sum (a one-node
                                  // cell's mean is its sum; every cell's circulation is a sum)
@@ -360,6 +352,12 @@ int ov_upload_member_tables(ov_ctx *c);
 int ov_move_device_slots(ov_ctx *c, const std::vector<Member> &old);
 void ov_tree_free(TreeBuf &t);
 int ov_tree_build(ov_ctx *c, const NodeArrays &na, cudaStream_t s);
+// Evaluations that take the split walk with the integer-mantissa law:
+// OV_PREC_DD always, OV_PREC_FP64 unless every test is to run in FP64.
+inline bool ov_split_walk(const ov_ctx *c, int precision)
+{
+    return precision == OV_PREC_DD || (precision == OV_PREC_FP64 && c->walk == OV_WALK_SPLIT);
+}
 // Unit of the integer law's coordinates: grid step / 2^bits, every separation
 // below 2^61 units (a box's grid leaves two periods of room, a spherical
 // section's none).

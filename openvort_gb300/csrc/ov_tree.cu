@@ -427,26 +427,6 @@ __device__ __forceinline__ void write_cell32(Cell32 *out, int ci, const double c
     o[2] = make_float4((float)q[0], (float)q[1], (float)q[2], lm32);
 }
 
-// Double-single view for the OV_PREC_DD law: the centre of mass as its grid
-// part (exact in FP32) plus the rest (exact in FP64) as hi + lo floats, the
-// circulation as hi + lo.
-__device__ __forceinline__ void write_cellff(CellFF *out, int ci, const double c[3], const double q[3], double h,
-                                             double inv_h)
-{
-    CellFF o;
-    for (int a = 0; a < 3; ++a) {
-        const double G = rint(c[a] * inv_h) * h;
-        const double f = c[a] - G;
-        o.g[a] = (float)G;
-        o.fh[a] = (float)f;
-        o.fl[a] = (float)(f - (double)o.fh[a]);
-        o.qh[a] = (float)q[a];
-        o.ql[a] = (float)(q[a] - (double)o.qh[a]);
-    }
-    o.pad = 0;
-    out[ci] = o;
-}
-
 // Fixed-point view for the FP64 path's integer law (ov_fxlaw.cuh): centre of
 // mass and circulation in units 1 / fx_inv, the circulation left-normalised.
 __device__ __forceinline__ void write_cellfx(CellFX *out, int ci, const double c[3], const double q[3], double fx_inv)
@@ -483,11 +463,9 @@ __device__ __forceinline__ void write_cellfx(CellFX *out, int ci, const double c
 }
 
 // What the traversals read of a cell once its sums are known: the means and
-// the circulation in the FP64 cell, the FP32, double-single and fixed-point
-// views.
+// the circulation in the FP64 cell, the FP32 and fixed-point views.
 struct CellViews {
     Cell32 *c32;
-    CellFF *cff;
     CellFX *cfx;
     double fx_inv;
     double h, inv_h, theta;
@@ -496,7 +474,7 @@ struct CellViews {
 };
 
 // Write a cell whole (64 bytes) once its sums are known: the means and the
-// circulation, Lm, successor and count, then the FP32 and double-single
+// circulation, Lm, successor and count, then the FP32 and fixed-point
 // views the traversals read.
 // (The mean of a one-node cell is its sum: a product with 1.0.  1 / count
 // comes from a table of the rounded quotients for the usual counts.)
@@ -519,7 +497,6 @@ __device__ __forceinline__ void store_cell(Cell64 *cells, int ci, const double s
         const float lm32 = v.lev_tab ? v.lev_tab[TREE_LV_SLOTS + lev] : __double2float_ru(lm);
         write_cell32(v.c32, ci, c, q, thr, lm32, next, v.h, v.inv_h);
     }
-    if (v.cff) write_cellff(v.cff, ci, c, q, v.h, v.inv_h);
     if (v.cfx) write_cellfx(v.cfx, ci, c, q, v.fx_inv);
 }
 
@@ -891,7 +868,6 @@ __global__ void k_root(const int *__restrict__ order, const int *__restrict__ ce
     if (views.c32)
         write_cell32(views.c32, root, c, q, cell_thr(r.lm, views.theta), __double2float_ru(r.lm), r.next, views.h,
                      views.inv_h);
-    if (views.cff) write_cellff(views.cff, root, c, q, views.h, views.inv_h);
     if (views.cfx) write_cellfx(views.cfx, root, c, q, views.fx_inv);
 }
 
@@ -901,16 +877,15 @@ int ov_tree_reserve_cells(ov_ctx *c, int cells)
 {
     TreeBuf &t = c->tree;
     if (t.cap_cells >= cells && t.cells) return OV_OK;
-    void *ptrs[] = {t.cells, t.cells32, t.cellsff, t.cellsfx, t.psum, t.first, t.lvl_list, t.lvl8};
+    void *ptrs[] = {t.cells, t.cells32, t.cellsfx, t.psum, t.first, t.lvl_list, t.lvl8};
     for (void *p : ptrs)
         if (p) cudaFree(p);
-    t.cells = nullptr; t.cells32 = nullptr; t.cellsff = nullptr; t.cellsfx = nullptr; t.first = t.lvl_list = nullptr;
+    t.cells = nullptr; t.cells32 = nullptr; t.cellsfx = nullptr; t.first = t.lvl_list = nullptr;
     t.psum = nullptr;
     t.lvl8 = nullptr;
     t.cap_cells = 0;
     OV_ALLOC(c, cudaMalloc(&t.cells, (size_t)cells * sizeof(Cell64)));
     OV_ALLOC(c, cudaMalloc(&t.cells32, (size_t)cells * sizeof(Cell32)));
-    OV_ALLOC(c, cudaMalloc(&t.cellsff, (size_t)cells * sizeof(CellFF)));
     OV_ALLOC(c, cudaMalloc(&t.cellsfx, (size_t)cells * sizeof(CellFX)));
     OV_ALLOC(c, cudaMalloc(&t.psum, (size_t)cells * 3 * 8));
     OV_ALLOC(c, cudaMalloc(&t.lvl8, (size_t)cells));
@@ -959,7 +934,7 @@ int ov_tree_reserve(ov_ctx *c, int cap)
 void ov_tree_free(TreeBuf &t)
 {
     void *ptrs[] = {t.keys, t.keys_alt, t.order, t.order_alt, t.torder, t.cpl, t.ncell_at, t.cell_off, t.scan_tmp,
-                    t.sort_hist, t.cells, t.cells32, t.cellsff, t.cellsfx, t.psum, t.first, t.lvl_list, t.lvl8, t.lvl_cnt, t.nm, t.lev_tab, t.inv_count,
+                    t.sort_hist, t.cells, t.cells32, t.cellsfx, t.psum, t.first, t.lvl_list, t.lvl8, t.lvl_cnt, t.nm, t.lev_tab, t.inv_count,
                     t.counters, t.tt};
     for (void *p : ptrs)
         if (p) cudaFree(p);
@@ -1034,8 +1009,7 @@ int ov_tree_build(ov_ctx *c, const NodeArrays &na, cudaStream_t s)
     CellViews views;
     const bool fp32_view = c->precision == OV_PREC_MIXED || c->precision == OV_PREC_DD || c->walk == OV_WALK_SPLIT;
     views.c32 = fp32_view ? t.cells32 : nullptr;
-    views.cff = c->precision == OV_PREC_DD ? t.cellsff : nullptr;
-    views.cfx = c->precision != OV_PREC_MIXED && c->walk == OV_WALK_SPLIT ? t.cellsfx : nullptr;
+    views.cfx = ov_split_walk(c, c->precision) ? t.cellsfx : nullptr;
     views.fx_inv = ldexp(1.0 / c->grid_h, ov_fx_bits(c));
     views.h = c->grid_h;
     views.inv_h = 1.0 / c->grid_h;

@@ -43,8 +43,7 @@ struct VelArgs {
     int S;                  // sub-walks per query point (FP64 split walk of a small tangle), else 1
     const Cell64 *cells;
     const Cell32 *cells32;
-    const CellFF *cellsff;      // OV_PREC_DD: double-single cell data
-    const CellFX *cellsfx;      // FP64 split walk: fixed-point cell data
+    const CellFX *cellsfx;      // split walk: fixed-point cell data
     double fx_inv;              // 1 / its unit (a power of two)
     const double *x, *y, *z, *tx, *ty, *tz, *nx, *ny, *nz;
     double *vx, *vy, *vz, *sx, *sy, *sz;
@@ -59,7 +58,6 @@ struct VelArgs {
     float shift_g[OV_MAX_IMAGES][3], shift_f[OV_MAX_IMAGES][3];   // L*shift split on the grid
     int cap;                // node slots (bounds checks)
     float th2f, near2f, f4pif;   // theta^2, near-field radius^2, KAPPA/4/pi in FP32
-    float f4pi_h, f4pi_l;        // KAPPA/4/pi in double-single
     double near2;           // mixed path: squared near-field radius
     unsigned long long *stat;
     unsigned *node_counts;  // when set: visits[cap], then accepts[cap], per target slot
@@ -883,11 +881,6 @@ __device__ __forceinline__ ff ff_mulf(ff x, float f)
     e = __fmaf_rn(x.lo, f, e);
     return ff_fast(p, e);
 }
-__device__ __forceinline__ ff ff_from(double v)
-{
-    const float h = (float)v;
-    return ff{h, (float)(v - (double)h)};
-}
 // 1/sqrt(x), x > 0: y0 from the hardware, then y = y0 + y0 (1 - x y0^2) / 2.
 // 1 - x y0^2 is of the order of y0's error: its leading part 1 - hi is exact
 // and the rest needs float precision only.
@@ -907,10 +900,6 @@ __device__ __forceinline__ ff ff_rcp(ff x)
     return ff_fast(y0, __fmul_rn(y0, r));
 }
 
-// One accepted cell in double-single: the segment law for R = COM - q,
-// Rp1 = R + circulation (sc = f4pi (1/|R| + 1/|Rp1|) / (|R| |Rp1| + R.Rp1),
-// w = (R x circulation) sc), added into the double-single sums acc[3].  The
-// query point is split like the cell: grid part gq (exact) plus fq.
 // The segment law for R (start - query) and S (segment vector) in
 // double-single: w = (R x S) f4pi (1/|R| + 1/|R+S|) / (|R| |R+S| + R.(R+S)).
 __device__ __forceinline__ void ff_segment(const ff R[3], const ff S[3], ff f4pi, ff w[3])
@@ -929,39 +918,8 @@ __device__ __forceinline__ void ff_segment(const ff R[3], const ff S[3], ff f4pi
     for (int a = 0; a < 3; ++a) w[a] = ff_mul(x[a], sc);
 }
 
-__device__ __forceinline__ void ff_law(const CellFF *cp, const float gq[3], const ff fq[3], ff f4pi, ff acc[3])
-{
-    const float4 *c4 = reinterpret_cast<const float4 *>(cp);
-    const float4 A = __ldg(c4), B = __ldg(c4 + 1), Cc = __ldg(c4 + 2), D = __ldg(c4 + 3);
-    // A = (g0, g1, g2, fh0)  B = (fh1, fh2, fl0, fl1)  Cc = (fl2, qh0, qh1, qh2)  D = (ql0, ql1, ql2, -)
-    const float gc[3] = {A.x, A.y, A.z};
-    const ff fc[3] = {ff{A.w, B.z}, ff{B.x, B.w}, ff{B.y, Cc.x}};
-    const ff q[3] = {ff{Cc.y, D.x}, ff{Cc.z, D.y}, ff{Cc.w, D.z}};
-    ff R[3], P[3];
-    for (int a = 0; a < 3; ++a) {
-        // grid parts differ exactly; the rest in double-single
-        R[a] = ff_add_f(ff_sub(fc[a], fq[a]), __fsub_rn(gc[a], gq[a]));
-        P[a] = ff_add(R[a], q[a]);
-    }
-    const ff lR2 = ff_add_sloppy(ff_add_sloppy(ff_mul(R[0], R[0]), ff_mul(R[1], R[1])), ff_mul(R[2], R[2]));
-    const ff lp2 = ff_add_sloppy(ff_add_sloppy(ff_mul(P[0], P[0]), ff_mul(P[1], P[1])), ff_mul(P[2], P[2]));
-    const ff dot = ff_add(ff_add(ff_mul(R[0], P[0]), ff_mul(R[1], P[1])), ff_mul(R[2], P[2]));
-    const ff ra = ff_rsqrt(lR2), rb = ff_rsqrt(lp2);
-    const ff ab = ff_mul(ra, rb);
-    const ff den = ff_add_f(ff_mul(dot, ab), 1.0f);
-    const ff sc = ff_mul(ff_mul(ff_mul(f4pi, ff_add_sloppy(ra, rb)), ab), ff_rcp(den));
-    const ff w[3] = {ff_sub(ff_mul(R[1], q[2]), ff_mul(R[2], q[1])), ff_sub(ff_mul(R[2], q[0]), ff_mul(R[0], q[2])),
-                     ff_sub(ff_mul(R[0], q[1]), ff_mul(R[1], q[0]))};
-    for (int a = 0; a < 3; ++a) acc[a] = ff_add_sloppy(acc[a], ff_mul(w[a], sc));
-}
-
-
-// value of a (sum, compensation) pair: Kahan's sum - compensation, or a
-// double-single's hi + lo
-__device__ __forceinline__ double acc_value(float s, float c, bool dd)
-{
-    return dd ? (double)s + (double)c : (double)s - (double)c;
-}
+// value of a Kahan (sum, compensation) pair
+__device__ __forceinline__ double acc_value(float s, float c) { return (double)s - (double)c; }
 
 struct MixedAcc {
     float s0, s1, s2, c0, c1, c2;   // Kahan sums over every query point
@@ -971,15 +929,10 @@ struct MixedAcc {
 // One query point (g + f split, image j; j < 0 the node itself) for the 32
 // lanes of a warp.  Near-field leaves are appended to the lane's list
 // (cell, image) and evaluated in FP64 after all query points.
-template <bool DD>
 __device__ __forceinline__ void bh_query32(const VelArgs &a, const float g[3], const float f[3], const double p[3],
                                            int j, bool part, int root, int ncell, MixedAcc &m, int *near_list,
-                                           int &nnear,
-                                           double w64[3], bool &overflow, const float *gqq = nullptr,
-                                           const ff *qff = nullptr)
+                                           int &nnear, double w64[3], bool &overflow)
 // near_list: this lane's column of a shared [kNearCap][32] array, stride 32.
-// DD: accepted interactions in double-single at the query point qff, summed
-// into (m.s, m.c) as (hi, lo) pairs; the near field needs no FP64 then.
 {
     const float near2 = a.near2f;
     const float f4pi = a.f4pif;
@@ -1035,8 +988,8 @@ __device__ __forceinline__ void bh_query32(const VelArgs &a, const float g[3], c
                 const float nd = dot * ab;
                 // the common case in one test: no deferral, the filter passing clear of its band
                 bool defer = false, keep = true;
-                if (exact || (!DD && leaf && d2 < near2) || lp2 < d2hi || !(nd > 1e-8f + 4e-6f)) {
-                    defer = exact || (!DD && leaf && d2 < near2) || lp2 < d2hi || fabsf(nd - 1e-8f) < 4e-6f;
+                if (exact || (leaf && d2 < near2) || lp2 < d2hi || !(nd > 1e-8f + 4e-6f)) {
+                    defer = exact || (leaf && d2 < near2) || lp2 < d2hi || fabsf(nd - 1e-8f) < 4e-6f;
                     keep = nd >= 1e-8f;
                 }
                 if (defer) {
@@ -1055,19 +1008,11 @@ __device__ __forceinline__ void bh_query32(const VelArgs &a, const float g[3], c
                         }
                     }
                 } else if (keep) {
-                    if (DD) {
-                        ff acc[3] = {ff{m.s0, m.c0}, ff{m.s1, m.c1}, ff{m.s2, m.c2}};
-                        ff_law(a.cellsff + c, gqq, qff, ff{a.f4pi_h, a.f4pi_l}, acc);
-                        m.s0 = acc[0].hi; m.c0 = acc[0].lo;
-                        m.s1 = acc[1].hi; m.c1 = acc[1].lo;
-                        m.s2 = acc[2].hi; m.c2 = acc[2].lo;
-                    } else {
-                        const float sc = __fdividef(f4pi * (ra + rb) * ab, fmaf(dot, ab, 1.0f));
-                        // R x Rp1 = R x q
-                        p0 = fmaf(fmaf(R1, qz, -R2 * qy), sc, p0);
-                        p1 = fmaf(fmaf(R2, qx, -R0 * qz), sc, p1);
-                        p2 = fmaf(fmaf(R0, qy, -R1 * qx), sc, p2);
-                    }
+                    const float sc = __fdividef(f4pi * (ra + rb) * ab, fmaf(dot, ab, 1.0f));
+                    // R x Rp1 = R x q
+                    p0 = fmaf(fmaf(R1, qz, -R2 * qy), sc, p0);
+                    p1 = fmaf(fmaf(R2, qx, -R0 * qz), sc, p1);
+                    p2 = fmaf(fmaf(R0, qy, -R1 * qx), sc, p2);
                 }
                 resume = nxt;
             } else if (skip) {
@@ -1078,25 +1023,21 @@ __device__ __forceinline__ void bh_query32(const VelArgs &a, const float g[3], c
         }
         ++steps;
         if ((steps & 15) == 0) {   // warp-uniform
-            if (!DD) {
-                kahan_add(m.s0, m.c0, p0);
-                kahan_add(m.s1, m.c1, p1);
-                kahan_add(m.s2, m.c2, p2);
-                p0 = p1 = p2 = 0;
-            }
+            kahan_add(m.s0, m.c0, p0);
+            kahan_add(m.s1, m.c1, p1);
+            kahan_add(m.s2, m.c2, p2);
+            p0 = p1 = p2 = 0;
             if (steps > guard_max) { overflow = true; break; }
         }
         c = __any_sync(0xffffffffu, open) ? c + 1 : nxt;
     }
-    if (!DD) {
-        kahan_add(m.s0, m.c0, p0);
-        kahan_add(m.s1, m.c1, p1);
-        kahan_add(m.s2, m.c2, p2);
-    }
+    kahan_add(m.s0, m.c0, p0);
+    kahan_add(m.s1, m.c1, p1);
+    kahan_add(m.s2, m.c2, p2);
     m.nstep += steps;
 }
 
-template <int W, int HI, bool DD>
+template <int W, int HI>
 __global__ void __launch_bounds__(32 * W, (min_blocks_mixed<W, HI>())) k_vel_mixed(VelArgs a,
                                                                                   double *__restrict__ part_out)
 {
@@ -1153,33 +1094,15 @@ __global__ void __launch_bounds__(32 * W, (min_blocks_mixed<W, HI>())) k_vel_mix
                 }
                 MixedAcc mr = {0, 0, 0, 0, 0, 0, 0u, 0u, 0u, 0u, 0u};
                 double wr[3] = {0, 0, 0};   // FP64 terms of this image when the near list is full
-                ff qr[3];
-                for (int ax = 0; ax < 3; ++ax) qr[ax] = ff_from(q[ax] - rint(q[ax] * a.inv_h) * a.grid_h);
-                bh_query32<DD>(a, g, f, p, j, part, w.root, w.end, mr, near_list, nnear, wr, overflow, g, qr);
-                double v[3] = {acc_value(mr.s0, mr.c0, DD) + wr[0], acc_value(mr.s1, mr.c1, DD) + wr[1],
-                               acc_value(mr.s2, mr.c2, DD) + wr[2]};
+                bh_query32(a, g, f, p, j, part, w.root, w.end, mr, near_list, nnear, wr, overflow);
+                double v[3] = {acc_value(mr.s0, mr.c0) + wr[0], acc_value(mr.s1, mr.c1) + wr[1],
+                               acc_value(mr.s2, mr.c2) + wr[2]};
                 for (int r = 0; r < a.geo.nreflect[j]; ++r) mirror_vec(a.geo.reflect[j][r], v);
                 img64[0] += v[0]; img64[1] += v[1]; img64[2] += v[2];
                 m.nvis += mr.nvis; m.nacc += mr.nacc; m.nstep += mr.nstep; m.nfb += mr.nfb; m.nnear += mr.nnear;
                 continue;
             }
-            if (DD) {
-                // the query point split as the cells are: the grid part exact, the rest
-                // (exact in FP64) in double-single
-                double q[3];
-                if (j < 0) { q[0] = p[0]; q[1] = p[1]; q[2] = p[2]; }
-                else image_point(a.geo, j, p, q);
-                float gq[3];
-                ff qf[3];
-                for (int ax = 0; ax < 3; ++ax) {
-                    const double G = rint(q[ax] * a.inv_h) * a.grid_h;
-                    gq[ax] = (float)G;
-                    qf[ax] = ff_from(q[ax] - G);
-                }
-                bh_query32<DD>(a, g, f, p, j, part, w.root, w.end, m, near_list, nnear, w64, overflow, gq, qf);
-            } else {
-                bh_query32<DD>(a, g, f, p, j, part, w.root, w.end, m, near_list, nnear, w64, overflow);
-            }
+            bh_query32(a, g, f, p, j, part, w.root, w.end, m, near_list, nnear, w64, overflow);
         }
         // deferred near-field interactions, all lanes together
         for (int i = 0; i < nnear && i < kNearCap; ++i) {
@@ -1195,9 +1118,9 @@ __global__ void __launch_bounds__(32 * W, (min_blocks_mixed<W, HI>())) k_vel_mix
             w64[0] += wv[0] * a.f4pi; w64[1] += wv[1] * a.f4pi; w64[2] += wv[2] * a.f4pi;
         }
         __syncwarp();   // the list is rewritten by the next item
-        double bh[3] = {acc_value(m.s0, m.c0, DD) + w64[0] + img64[0],
-                        acc_value(m.s1, m.c1, DD) + w64[1] + img64[1],
-                        acc_value(m.s2, m.c2, DD) + w64[2] + img64[2]};
+        double bh[3] = {acc_value(m.s0, m.c0) + w64[0] + img64[0],
+                        acc_value(m.s1, m.c1) + w64[1] + img64[1],
+                        acc_value(m.s2, m.c2) + w64[2] + img64[2]};
         if (valid) {
             const size_t cap = (size_t)a.cap;
             for (int ax = 0; ax < 3; ++ax) {
@@ -1435,8 +1358,8 @@ __global__ void __launch_bounds__(32 * W, (min_blocks_mixp<W, R>())) k_vel_mixp(
         __syncwarp();   // the list is rewritten by the next item
         if (valid) {
             const size_t cap = (size_t)a.cap;
-            const double bh[3] = {acc_value(m.s0, m.c0, false) + w64[0], acc_value(m.s1, m.c1, false) + w64[1],
-                                  acc_value(m.s2, m.c2, false) + w64[2]};
+            const double bh[3] = {acc_value(m.s0, m.c0) + w64[0], acc_value(m.s1, m.c1) + w64[1],
+                                  acc_value(m.s2, m.c2) + w64[2]};
             for (int ax = 0; ax < 3; ++ax) {
                 part_out[((size_t)(2 * w.grp) * 3 + ax) * cap + tix] = bh[ax];
                 part_out[((size_t)(2 * w.grp + 1) * 3 + ax) * cap + tix] = 0.0;
@@ -1469,7 +1392,7 @@ __global__ void __launch_bounds__(32 * W, (min_blocks_mixp<W, R>())) k_vel_mixp(
     }
 }
 
-// ------------------------------------------- FP64 path, split walk (default)
+// -------------------------- FP64 path, split walk (default), and OV_PREC_DD
 // The walk (distance and opening tests) runs in FP32 on the grid-split cells
 // exactly as the mixed traversal's, with the FP64 test inside the guard
 // bands, so every lane accepts, skips and opens the cells the FP64 walk
@@ -1818,7 +1741,7 @@ int ov_query_groups(ov_ctx *c)
     int maxg = c->geo.n_img + 1;
     if (c->tune.groups > 0) return std::min(c->tune.groups, std::min(maxg, 27));
     int warps = (c->cap + 31) / 32;
-    const bool split = c->precision == OV_PREC_FP64 && c->walk == OV_WALK_SPLIT;
+    const bool split = ov_split_walk(c, c->precision);
     const int per_sm = split ? 400 : 32, gmax = split ? 27 : 8;
     int G = (per_sm * c->sm_count + warps - 1) / warps;
     G = G < 1 ? 1 : (G > gmax ? gmax : G);
@@ -1834,7 +1757,6 @@ VelArgs make_args(ov_ctx *c, const NodeArrays &na, double t, unsigned long long 
     a.counters = c->tree.counters;
     a.cells = c->tree.cells;
     a.cells32 = c->tree.cells32;
-    a.cellsff = c->tree.cellsff;
     a.cellsfx = c->tree.cellsfx;
     a.fx_inv = c->grid_h > 0 ? ldexp(1.0 / c->grid_h, ov_fx_bits(c)) : 0;
     a.x = na.x; a.y = na.y; a.z = na.z;
@@ -1875,8 +1797,6 @@ VelArgs make_args(ov_ctx *c, const NodeArrays &na, double t, unsigned long long 
     a.th2f = (float)(a.prm.theta * a.prm.theta);
     a.near2f = (float)a.near2;
     a.f4pif = (float)a.f4pi;
-    a.f4pi_h = (float)a.f4pi;
-    a.f4pi_l = (float)(a.f4pi - (double)a.f4pi_h);
     a.node_counts = nullptr;
     a.cell_first = c->geo.sph ? nullptr : c->tree.first;
     a.keys = c->tree.keys;
@@ -1909,7 +1829,7 @@ constexpr int kSubWalkSlots = 8192;
 static int sub_walks_for(int cap) { return cap <= 2048 ? 32 : (cap <= kSubWalkSlots ? 8 : 1); }
 static int ov_sub_walks(const ov_ctx *c, int precision)
 {
-    return precision == OV_PREC_FP64 && c->walk == OV_WALK_SPLIT ? sub_walks_for(c->cap) : 1;
+    return ov_split_walk(c, precision) ? sub_walks_for(c->cap) : 1;
 }
 
 int ov_reserve_velocity_scratch(ov_ctx *c)
@@ -1944,26 +1864,21 @@ template <int R> static VelKernel mixp_kernel(int warps)
     return k_vel_mixp<4, R>;
 }
 
-static VelKernel vel_kernel(int precision, int walk, int warps, int hi_occ, bool mirror)
+static VelKernel vel_kernel(int precision, bool split, int warps, int hi_occ, bool mirror)
 {
     if (precision == OV_PREC_MIXED) {
         if (hi_occ >= 2 && !mirror) return hi_occ == 2 ? mixp_kernel<0>(warps)
                                          : (hi_occ == 3 ? mixp_kernel<80>(warps) : mixp_kernel<64>(warps));
         if (hi_occ) {
-            if (warps == 2) return k_vel_mixed<2, 1, false>;
-            if (warps == 8) return k_vel_mixed<8, 1, false>;
-            return k_vel_mixed<4, 1, false>;
+            if (warps == 2) return k_vel_mixed<2, 1>;
+            if (warps == 8) return k_vel_mixed<8, 1>;
+            return k_vel_mixed<4, 1>;
         }
-        if (warps == 2) return k_vel_mixed<2, 0, false>;
-        if (warps == 8) return k_vel_mixed<8, 0, false>;
-        return k_vel_mixed<4, 0, false>;
+        if (warps == 2) return k_vel_mixed<2, 0>;
+        if (warps == 8) return k_vel_mixed<8, 0>;
+        return k_vel_mixed<4, 0>;
     }
-    if (precision == OV_PREC_DD) {
-        if (warps == 2) return k_vel_mixed<2, 0, true>;
-        if (warps == 8) return k_vel_mixed<8, 0, true>;
-        return k_vel_mixed<4, 0, true>;
-    }
-    if (walk == OV_WALK_SPLIT) {
+    if (split) {
         if (warps == 2) return k_vel_split<2>;
         if (warps == 8) return k_vel_split<8>;
         return k_vel_split<4>;
@@ -1977,7 +1892,7 @@ static VelKernel vel_kernel(int precision, int walk, int warps, int hi_occ, bool
 // block of 8 warps needs the opt-in above 48 KB.
 static size_t list_bytes(const ov_ctx *c, int precision, int warps)
 {
-    if (precision != OV_PREC_FP64 || c->walk != OV_WALK_SPLIT) return 0;
+    if (!ov_split_walk(c, precision)) return 0;
     if (warps == 8)
         cudaFuncSetAttribute(k_vel_split<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * (int)sizeof(WarpLists));
     return warps * sizeof(WarpLists);
@@ -1987,7 +1902,7 @@ static size_t list_bytes(const ov_ctx *c, int precision, int warps)
 // every SM, but no more blocks than there can be work items.
 int ov_traversal_blocks(ov_ctx *c, int precision, int warps, int *per_sm)
 {
-    VelKernel k = vel_kernel(precision, c->walk, warps, c->tune.hi_occ, has_mirror_images(c->geo));
+    VelKernel k = vel_kernel(precision, ov_split_walk(c, precision), warps, c->tune.hi_occ, has_mirror_images(c->geo));
     int occ = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, 32 * warps, list_bytes(c, precision, warps)) !=
             cudaSuccess || occ < 1) {
@@ -2029,7 +1944,7 @@ int ov_launch_velocities(ov_ctx *c, const NodeArrays &na, double t, int precisio
         a.node_counts = c->d_node_counts;
     }
     OV_CUDA(c, cudaMemsetAsync(a.work, 0, sizeof(int), s));
-    vel_kernel(precision, c->walk, warps, c->tune.hi_occ, has_mirror_images(c->geo))<<<
+    vel_kernel(precision, ov_split_walk(c, precision), warps, c->tune.hi_occ, has_mirror_images(c->geo))<<<
         blocks, 32 * warps, list_bytes(c, precision, warps), s>>>(a, c->part);
     if (a.S > 1) {
         const long long threads = 6LL * c->cap * a.G;
@@ -3284,7 +3199,7 @@ __global__ void __launch_bounds__(128) k_sph_query_mixed(SphArgs s, double *__re
     double w64[3] = {0, 0, 0};
     int nnear = 0;
     bool overflow = false;
-    bh_query32<false>(a, g, f, qp, -1, go, root, end, acc, near_list, nnear, w64, overflow);
+    bh_query32(a, g, f, qp, -1, go, root, end, acc, near_list, nnear, w64, overflow);
     for (int i = 0; i < nnear && i < kNearCap; ++i) {
         const int e = near_list[32 * i];
         const int c = e >> 5;
