@@ -42,8 +42,13 @@ struct alignas(16) CellFX {
 };
 constexpr int kFxNone = -1, kFxZero = -2;
 constexpr int kFxMaxShift = 9;     // |R| below 2^(60 - 9) units: FP64 law
-constexpr int kFxUnit = -105;      // terms add up in units 2^kFxUnit / u
+// Terms add up in units 2^kFxUnit / u.  A term's error is about 2^-8 units (the
+// aligned quotient's last bit), and terms with a quotient above 2^63 units, the
+// nearest, are left to the FP64 law: the unit of a tree's sums (2,000 terms)
+// sends it a handful, that of direct sums (10^6 terms) a few hundred.
+constexpr int kFxUnit = -105, kFxUnitDirect = -110;
 constexpr int kFxTerms = 31;       // terms a sum holds: each is at most 2^58 units
+constexpr double kFxLimit = 2305843009213693952.0;   // 2^61: coordinates a view holds
 
 #if defined(__CUDA_ARCH__)
 #define FX_INLINE __device__ __forceinline__
@@ -134,10 +139,36 @@ FX_INLINE int64_t fx_mulhi(int64_t a, int64_t b)
     return (int64_t)fx_madu(ah, bh, mid >> 32);
 }
 
+// The view of a cell or segment from its coordinates in units u; fits: they
+// are below 2^61.
+FX_INLINE CellFX fx_cell(const int64_t c[3], const int64_t s[3], bool fits)
+{
+    CellFX o;
+    uint64_t m = 0;
+    for (int i = 0; i < 3; ++i) m |= (uint64_t)(s[i] < 0 ? -s[i] : s[i]);
+    const int hi = fx_clz((unsigned)(m >> 32)), lo = fx_clz((unsigned)m);
+    o.e = !fits ? kFxNone : (m ? (m >> 32 ? hi : 32 + lo) - 3 : kFxZero);
+    o.n = 0;
+    int64_t low = 0;
+    for (int i = 0; i < 3; ++i) {
+        o.c[i] = c[i];
+        const fx_split p = fx_parts(o.e > 0 ? (int64_t)((uint64_t)s[i] << o.e) : s[i]);
+        o.sh[i] = p.h;
+        o.sl[i] = p.l;
+        o.n = fx_mad(p.h, p.h, o.n);
+        low = fx_mad(p.h, p.l, low);
+    }
+    o.n += low >> 31;
+    o.pad = 0;
+    return o;
+}
+
 // Adds the law's term for cell c seen from q (units u) to sum where `take` is
 // set and the law can decide; returns that (no branches: what is left to the
-// FP64 law is rare).
-FX_INLINE bool fx_law(const CellFX &c, const int64_t q[3], bool take, fx_sum sum[3])
+// FP64 law is rare).  mag, when given, gains a bound on the term's
+// magnitude (over the components, in the sum's units, to FP32 precision).
+template <int Unit = kFxUnit>
+FX_INLINE bool fx_law(const CellFX &c, const int64_t q[3], bool take, fx_sum sum[3], float *mag = nullptr)
 {
     int64_t R[3];
     unsigned top = 0;
@@ -183,9 +214,11 @@ FX_INLINE bool fx_law(const CellFX &c, const int64_t q[3], bool take, fx_sum sum
     const int q2 = fx_int((float)(int)(e2 >> 4) * (y * 1048576.0f));
     const int64_t Q = fx_mad(q1, 65536, q2) + ((int64_t)q0 << 32);
     // the term is (R x S) / 2^64 Q / 2^64 2^ex, ex = lg + lh - ls + 2 s - e - 122
-    const int down = kFxUnit + 122 + ls + c.e - lg - lh - 2 * s;
+    const int down = Unit + 122 + ls + c.e - lg - lh - 2 * s;
     ok = ok && down >= 0;
     const fx_split k = fx_parts(ok ? fx_shr(Q, down) : 0);
+    // (p.h + 1) 2^32 |k| / 2^64 bounds a component's term
+    const float size = mag ? fmaf((float)k.h, 1.0f, (float)k.l * 2.3283064e-10f) : 0.0f;
     for (int i = 0; i < 3; ++i) {
         const int u = i == 2 ? 0 : i + 1, v = i == 0 ? 2 : i - 1;
         int64_t x = fx_mul(r[u].h, c.sl[v]);
@@ -197,6 +230,7 @@ FX_INLINE bool fx_law(const CellFX &c, const int64_t q[3], bool take, fx_sum sum
         const fx_split p = fx_parts(x);
         int64_t low = fx_mad(p.h, k.l, fx_hi(fx_mul(p.l, k.l)));
         low = fx_mad(p.l, k.h, low);
+        if (mag) *mag = fmaf(fabsf((float)p.h) + 1.0f, size, *mag);
         fx_add(sum[i], fx_mad(p.h, k.h, fx_hi(low)), (unsigned)low);
     }
     return ok;

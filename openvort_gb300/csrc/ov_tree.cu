@@ -431,31 +431,15 @@ __device__ __forceinline__ void write_cell32(Cell32 *out, int ci, const double c
 // mass and circulation in units 1 / fx_inv, the circulation left-normalised.
 __device__ __forceinline__ void write_cellfx(CellFX *out, int ci, const double c[3], const double q[3], double fx_inv)
 {
-    CellFX o;
-    uint64_t m = 0;
     bool fits = true;
-    int64_t s[3];
+    int64_t x[3], s[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        const double x = c[a] * fx_inv, y = q[a] * fx_inv;
-        fits = fits && fabs(x) < 2305843009213693952.0 && fabs(y) < 2305843009213693952.0;   // 2^61
-        o.c[a] = __double2ll_rn(x);
-        s[a] = __double2ll_rn(y);
-        m |= (uint64_t)(s[a] < 0 ? -s[a] : s[a]);
+        fits = fits && fabs(c[a] * fx_inv) < kFxLimit && fabs(q[a] * fx_inv) < kFxLimit;
+        x[a] = __double2ll_rn(c[a] * fx_inv);
+        s[a] = __double2ll_rn(q[a] * fx_inv);
     }
-    o.e = fits ? (m ? __clzll((long long)m) - 3 : kFxZero) : kFxNone;
-    o.n = 0;
-    int64_t low = 0;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        const fx_split p = fx_parts(o.e > 0 ? (int64_t)((uint64_t)s[a] << o.e) : s[a]);
-        o.sh[a] = p.h;
-        o.sl[a] = p.l;
-        o.n += fx_mul(p.h, p.h);
-        low += fx_mul(p.h, p.l);
-    }
-    o.n += low >> 31;
-    o.pad = 0;
+    const CellFX o = fx_cell(x, s, fits);
     const int4 *src = reinterpret_cast<const int4 *>(&o);
     int4 *dst = reinterpret_cast<int4 *>(out + ci);
 #pragma unroll

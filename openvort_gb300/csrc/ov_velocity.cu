@@ -1440,7 +1440,7 @@ __device__ __forceinline__ double3 run_list(const CellFX *cells, const Cell64 *c
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
         const double x = L.q[i][lane] * fx_inv;
-        in_range = in_range && fabs(x) < 2305843009213693952.0;   // 2^61
+        in_range = in_range && fabs(x) < kFxLimit;
         q[i] = __double2ll_rn(x);
     }
     double v[3] = {0.0, 0.0, 0.0};
@@ -2153,10 +2153,10 @@ constexpr int kRecVals = 7;   // 3 sums, FP32 magnitude, 3 spare (|FP64 terms|)
 template <int MODE, bool MIRROR>
 __global__ void __launch_bounds__(kRecThreads, 3) k_rec_sums(RecArgs r, const int *__restrict__ nodes, int n,
                                                           int span, int max_chunks, double *__restrict__ part)
-// MODE: 0 FP32 far / FP64 near, 1 all FP64, 2 double-single far / FP64 near.
+// MODE: 0 FP32 far / FP64 near, 2 double-single far / FP64 near (all in FP64:
+// k_direct_fx).
 // MIRROR: the image set has mirror images (their query points in FP64).
 {
-    constexpr int force64 = MODE;
     // split query points (self, then images): (g, mirror flag), (f, 0), (f's rest, 0)
     __shared__ float4 s_q[OV_MAX_IMAGES + 1][3];
     // FP32 mode: the negated query points in pairs (0,1), (2,3), ... for the
@@ -2199,7 +2199,7 @@ __global__ void __launch_bounds__(kRecThreads, 3) k_rec_sums(RecArgs r, const in
             }
         }
         // mirror images (reflected query points): FP64 unless double-single
-        const float mirror = (force64 != 2 && j >= 0 && r.geo.nreflect[j] > 0) ? 1.0f : 0.0f;
+        const float mirror = (MODE != 2 && j >= 0 && r.geo.nreflect[j] > 0) ? 1.0f : 0.0f;
         s_q[threadIdx.x][0] = make_float4(g[0], g[1], g[2], mirror);
         s_q[threadIdx.x][1] = make_float4(f[0], f[1], f[2], 0.0f);
         s_q[threadIdx.x][2] = make_float4(fl[0], fl[1], fl[2], 0.0f);
@@ -2221,7 +2221,7 @@ __global__ void __launch_bounds__(kRecThreads, 3) k_rec_sums(RecArgs r, const in
         if (f < 0 || f >= r.cap) continue;
         float ag[3], af[3], sv[3];
         ff fa[3], S[3];   // mode 2: the start's rest and the segment vector in double-single
-        bool seg64 = force64 == 1;
+        bool seg64 = false;
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
             ag[a] = r.sp[(size_t)a * r.cap + m];
@@ -2352,7 +2352,7 @@ __global__ void __launch_bounds__(kRecThreads, 3) k_rec_sums(RecArgs r, const in
         for (; mask64; mask64 &= mask64 - 1) {
             const int j = __ffs(mask64) - 2;
             double w[3];
-            if (force64 == 1 ? rec_term64_fast(r, m, f, j, p, w) : rec_term64(r, m, f, j, p, w)) {
+            if (rec_term64(r, m, f, j, p, w)) {
                 d0 += w[0]; d1 += w[1]; d2 += w[2];
                 dabs += fabs(w[0]) + fabs(w[1]) + fabs(w[2]);
             }
@@ -2378,6 +2378,106 @@ __global__ void __launch_bounds__(kRecThreads, 3) k_rec_sums(RecArgs r, const in
         __syncthreads();
     }
     if (threadIdx.x < kRecVals) out[threadIdx.x] = red[threadIdx.x][0];
+}
+
+// The segments in fixed point for k_direct_fx: start, vector to the end moved
+// by a period toward it (seg_pwrap), zero where there is none.
+__global__ void k_segments_fx(RecArgs r, double fx_inv, CellFX *__restrict__ out)
+{
+    const int m = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m >= r.cap) return;
+    const int f = r.fwd[m];
+    const double s1[3] = {r.x[m], r.y[m], r.z[m]};
+    double s2[3] = {s1[0], s1[1], s1[2]};
+    if (f >= 0 && f < r.cap) {
+        s2[0] = r.x[f]; s2[1] = r.y[f]; s2[2] = r.z[f];
+        pwrap_dev(r.geo, s1, s2);
+    }
+    bool fits = true;
+    int64_t c[3], s[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        fits = fits && fabs(s1[a] * fx_inv) < kFxLimit && fabs(s2[a] * fx_inv) < kFxLimit;
+        c[a] = __double2ll_rn(s1[a] * fx_inv);
+        s[a] = __double2ll_rn(s2[a] * fx_inv) - c[a];
+        fits = fits && s[a] < (1ll << 61) && s[a] > -(1ll << 61);
+    }
+    out[m] = fx_cell(c, s, fits);
+}
+
+// FP64 direct sums in (node, segment chunk) blocks: each thread takes segments
+// of the chunk and, for each, every query point (the node and its images) by
+// the integer-mantissa law (ov_fxlaw.cuh); what that leaves to the FP64 law
+// after the loop.  Layout of part as k_rec_sums: the sums, then in [4] the sum
+// of the terms' magnitudes.
+// Integer pipe: 16 cycles an interaction and SM.  2,048 nodes of 32,768 with
+// 26 images: 34 ms, 303 with every term in FP64.
+__global__ void __launch_bounds__(kRecThreads, 3) k_direct_fx(RecArgs r, double fx_inv,
+                                                              const CellFX *__restrict__ seg,
+                                                              const int *__restrict__ nodes, int n, int span,
+                                                              int max_chunks, double *__restrict__ part)
+{
+    __shared__ int64_t s_q[OV_MAX_IMAGES + 1][3];
+    __shared__ bool s_in[OV_MAX_IMAGES + 1];
+    __shared__ double red[4][kRecThreads];
+    const int b = blockIdx.x, chunk = blockIdx.y;
+    if (b >= n) return;
+    const int k = nodes[b];
+    int lo, hi;
+    member_range(r, k, lo, hi);
+    const int m0 = lo + chunk * span, m1 = min(hi, m0 + span);
+    double *out = part + ((size_t)b * max_chunks + chunk) * kRecVals;
+    if (m0 >= m1 || k < 0 || k >= r.cap) {
+        if (threadIdx.x < kRecVals) out[threadIdx.x] = 0.0;
+        return;
+    }
+    const double p[3] = {r.x[k], r.y[k], r.z[k]};
+    const int nq = r.geo.n_img + 1;
+    if (threadIdx.x < nq) {
+        const int j = (int)threadIdx.x - 1;
+        double q[3];
+        if (j < 0) { q[0] = p[0]; q[1] = p[1]; q[2] = p[2]; }
+        else image_point(r.geo, j, p, q);
+        bool in = true;
+        for (int a = 0; a < 3; ++a) {
+            in = in && fabs(q[a] * fx_inv) < kFxLimit;
+            s_q[threadIdx.x][a] = __double2ll_rn(q[a] * fx_inv);
+        }
+        s_in[threadIdx.x] = in;
+    }
+    __syncthreads();
+    const double unit = ldexp(1.0, kFxUnitDirect) * fx_inv * r.f4pi;
+    double d[3] = {0, 0, 0}, dabs = 0;
+    for (int m = m0 + threadIdx.x; m < m1; m += blockDim.x) {
+        const int f = r.fwd[m];
+        if (f < 0 || f >= r.cap) continue;
+        const CellFX c = load_cellfx(seg + m);
+        const int first = (m == k || f == k) ? 1 : 0;   // the node's own segments: not at the primary point
+        fx_sum sum[3] = {{0, 0}, {0, 0}, {0, 0}};
+        float mag = 0;
+        unsigned mask64 = 0;
+#pragma unroll 1
+        for (int qi = first; qi < nq; ++qi)
+            if (!fx_law<kFxUnitDirect>(c, s_q[qi], s_in[qi], sum, &mag)) mask64 |= 1u << qi;
+        for (int a = 0; a < 3; ++a) d[a] = fma(fx_value(sum[a]), unit, d[a]);
+        dabs = fma((double)mag, unit, dabs);
+        for (; mask64 && c.e != kFxZero; mask64 &= mask64 - 1) {
+            double w[3];
+            if (rec_term64_fast(r, m, f, __ffs(mask64) - 2, p, w)) {
+                for (int a = 0; a < 3; ++a) d[a] += w[a];
+                dabs += fabs(w[0]) + fabs(w[1]) + fabs(w[2]);
+            }
+        }
+    }
+    for (int a = 0; a < 3; ++a) red[a][threadIdx.x] = d[a];
+    red[3][threadIdx.x] = dabs;
+    __syncthreads();
+    for (int off = blockDim.x / 2; off > 0; off >>= 1) {
+        if (threadIdx.x < off)
+            for (int v = 0; v < 4; ++v) red[v][threadIdx.x] += red[v][threadIdx.x + off];
+        __syncthreads();
+    }
+    if (threadIdx.x < kRecVals) out[threadIdx.x] = threadIdx.x < 3 ? red[threadIdx.x][0] : (threadIdx.x == 4 ? red[3][0] : 0.0);
 }
 
 // out[5 b + {0,1,2}] = sums over the chunks in order, out[5 b + 3] = bound on
@@ -2592,22 +2692,49 @@ int rec_reserve(ov_ctx *c, int n, int max_chunks)
     return OV_OK;
 }
 
+// FP64 sums of n nodes into rec_part: chunks of up to 8,192 segments, shorter
+// where few nodes would leave SMs without a block.
+int rec_launch_fx(ov_ctx *c, const RecArgs &ra, const int *d_nodes, int n, int *chunks)
+{
+    int maxcap = 1;
+    for (const Member &m : c->mem) maxcap = std::max(maxcap, c->mem.size() == 1 ? c->cap : m.cap);
+    const int most = std::max(1, (maxcap + kRecThreads - 1) / kRecThreads);
+    const int want = std::max((maxcap + 8191) / 8192, (8 * c->sm_count + n - 1) / n);
+    const int span = (maxcap + std::min(want, most) - 1) / std::min(want, most);
+    *chunks = (maxcap + span - 1) / span;
+    int r = rec_reserve(c, n, *chunks);
+    if (r) return r;
+    if (c->rec_seg_cap < c->cap) {
+        if (c->rec_seg) cudaFree(c->rec_seg);
+        c->rec_seg = nullptr;
+        c->rec_seg_cap = 0;
+        OV_ALLOC(c, cudaMalloc(&c->rec_seg, (size_t)c->cap * sizeof(CellFX)));
+        c->rec_seg_cap = c->cap;
+    }
+    const double fx_inv = ldexp(1.0 / c->grid_h, ov_fx_bits(c));
+    k_segments_fx<<<(c->cap + 255) / 256, 256, 0, c->stream>>>(ra, fx_inv, c->rec_seg);
+    k_direct_fx<<<dim3(n, *chunks), kRecThreads, 0, c->stream>>>(ra, fx_inv, c->rec_seg, d_nodes, n, span, *chunks,
+                                                                c->rec_part);
+    c->launches += 2;
+    return OV_OK;
+}
+
 // mode: 0 mixed (FP32 far, FP64 near), 1 FP64, 2 double-single far, FP64 near
 int rec_launch_sums(ov_ctx *c, const int *d_nodes, int n, int mode, double *out_host)
 {
     int maxcap = 0;
     for (const Member &m : c->mem) maxcap = std::max(maxcap, c->mem.size() == 1 ? c->cap : m.cap);
     const int span = 8192;
-    const int max_chunks = std::max(1, (maxcap + span - 1) / span);
+    int max_chunks = std::max(1, (maxcap + span - 1) / span);
     int r = rec_reserve(c, n, max_chunks);
     if (r) return r;
     RecArgs ra = make_rec_args(c);
     dim3 grid(n, max_chunks);
     bool mirror = false;
     for (int j = 0; j < c->geo.n_img; ++j) mirror = mirror || c->geo.nreflect[j] > 0;
-    if (mode == 1)
-        k_rec_sums<1, true><<<grid, kRecThreads, 0, c->stream>>>(ra, d_nodes, n, span, max_chunks, c->rec_part);
-    else if (mode == 2 && mirror)
+    if (mode == 1) {
+        if ((r = rec_launch_fx(c, ra, d_nodes, n, &max_chunks))) return r;
+    } else if (mode == 2 && mirror)
         k_rec_sums<2, true><<<grid, kRecThreads, 0, c->stream>>>(ra, d_nodes, n, span, max_chunks, c->rec_part);
     else if (mode == 2)
         k_rec_sums<2, false><<<grid, kRecThreads, 0, c->stream>>>(ra, d_nodes, n, span, max_chunks, c->rec_part);
@@ -2687,21 +2814,15 @@ extern "C" int ov_direct_sums_bounded(ov_ctx *c, const int *nodes, int n, int pr
 // then LIA, v_s and friction (k_direct_finish) into device arrays.
 int ov_direct_sum_chunked(ov_ctx *c, const int *nodes, int n, double *d_out_vel, double *d_out_vs, double t)
 {
-    int maxcap = 0;
-    for (const Member &m : c->mem) maxcap = std::max(maxcap, c->mem.size() == 1 ? c->cap : m.cap);
-    const int span = 8192, max_chunks = std::max(1, (maxcap + span - 1) / span);
-    int r = rec_reserve(c, n, max_chunks);
+    int r = rec_reserve(c, n, 1);
     if (r) return r;
     OV_CUDA(c, cudaMemcpyAsync(c->rec_nodes, nodes, (size_t)n * sizeof(int), cudaMemcpyHostToDevice, c->stream));
-    k_split<<<(c->cap + 255) / 256, 256, 0, c->stream>>>(c->node.x, c->node.y, c->node.z, c->cap, c->grid_h,
-                                                        1.0 / c->grid_h, c->rec_split);
-    RecArgs ra = make_rec_args(c);
-    k_rec_sums<1, true><<<dim3(n, max_chunks), kRecThreads, 0, c->stream>>>(ra, c->rec_nodes, n, span, max_chunks,
-                                                                      c->rec_part);
-    k_rec_finish<<<(n + 127) / 128, 128, 0, c->stream>>>(c->rec_part, n, max_chunks, c->rec_out);
+    int chunks = 0;
+    if ((r = rec_launch_fx(c, make_rec_args(c), c->rec_nodes, n, &chunks))) return r;
+    k_rec_finish<<<(n + 127) / 128, 128, 0, c->stream>>>(c->rec_part, n, chunks, c->rec_out);
     VelArgs a = make_args(c, c->node, t, nullptr);
     k_direct_finish<<<(n + 127) / 128, 128, 0, c->stream>>>(a, c->rec_nodes, n, c->rec_out, 5, d_out_vel, d_out_vs);
-    c->launches += 4;
+    c->launches += 2;
     OV_CUDA(c, cudaGetLastError());
     return OV_OK;
 }

@@ -33,28 +33,16 @@ int main(int argc, char **argv)
     long taken = 0, bad = 0;
     for (long it = 0; it < 400000; ++it) {
         const double d = 0x1p51 * pow(span, un()), mag = smax * pow(1e-4, un());
-        int64_t q[3], R[3], S[3];
-        CellFX c;
+        int64_t q[3], R[3], S[3], at[3];
         for (int i = 0; i < 3; ++i) {
             const int64_t mask = ~((1ll << zeros) - 1);
             q[i] = (int64_t)((un() - 0.5) * 0x1p60) & mask;
             R[i] = (int64_t)((2 * un() - 1) * d) & mask;
             S[i] = (int64_t)((2 * un() - 1) * d * mag) & mask;
-            c.c[i] = q[i] + R[i];
+            at[i] = q[i] + R[i];
         }
-        uint64_t m = 0;
-        for (int i = 0; i < 3; ++i) m |= (uint64_t)(S[i] < 0 ? -S[i] : S[i]);
-        if (!m) continue;
-        c.e = __builtin_clzll(m) - 3;
-        int64_t low = 0;
-        c.n = 0;
-        for (int i = 0; i < 3; ++i) {
-            const fx_split p = fx_parts((int64_t)((uint64_t)S[i] << c.e));
-            c.sh[i] = p.h; c.sl[i] = p.l;
-            c.n += fx_mul(p.h, p.h);
-            low += fx_mul(p.h, p.l);
-        }
-        c.n += low >> 31;
+        const CellFX c = fx_cell(at, S, true);
+        if (c.e < 0) continue;
         fx_sum w[3] = {{0, 0}, {0, 0}, {0, 0}};
         if (!fx_law(c, q, true, w)) {
             for (int i = 0; i < 3; ++i) bad += w[i].h != 0 || w[i].l != 0;   // left untouched
@@ -143,3 +131,25 @@ def test_split_walk_equals_fp64_walk(make, theta):
     per_node = np.linalg.norm(v - v64, axis=1) / np.linalg.norm(v64, axis=1)
     assert per_node.max() < 1e-10
     assert np.linalg.norm(v - v64) < 1e-12 * np.linalg.norm(v64)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("make,nodes", [
+    (lambda: W.random_walk_tangle(1, 7, D=0.1, seed=3), 7),              # fewer segments than threads
+    (lambda: W.random_walk_tangle(3, 257, D=0.1, seed=4), 1),            # one node: shortest chunks
+    (lambda: W.random_walk_tangle(70, 250, D=0.1, seed=5, n_images=6), 130),   # a ragged last chunk
+    (lambda: _close(600, 0.1, 1e-5, 6), 50),                              # nearly every segment left to FP64
+])
+def test_direct_sums_equal_fp64_terms(make, nodes):
+    """The direct sums' integer law against the allocation-free entry point,
+    which evaluates every term in FP64, at the FP64 parity tolerance."""
+    torch = pytest.importorskip("torch")
+    from tests._util import node_rel_err
+    from tests.test_zz_no_alloc import _Caller, _reference
+    ht = make()
+    p = W.config_params("rw")
+    ids = np.linspace(0, ht.n - 1, nodes).astype(np.int32)
+    (ref,) = _reference(ht, p, [ids])
+    got = _Caller(torch, ht, p).call(ids)
+    assert node_rel_err(got[0], ref[0]) < 1e-10
+    assert node_rel_err(got[1], ref[1]) < 1e-10
