@@ -163,7 +163,7 @@ static void release_buffers(ov_ctx *c)
     ov_tree_free(c->tree);
     void *dev[] = {c->fwd, c->rev, c->status, c->pin, c->dnodes, c->d_tid, c->d_qorder, c->d_tprm, c->d_mrange,
                    c->d_pairs, c->d_npairs, c->d_loop_off, c->d_loop_nodes, c->d_loop_buf, c->d_loop_cut,
-                   c->rec_nodes, c->rec_pair, c->rec_out, c->rec_corr, c->rec_part, c->rec_split, c->rec_seg, c->fft_buf,
+                   c->rec_nodes, c->rec_pair, c->rec_out, c->rec_corr, c->rec_part, c->rec_split, c->rec_seg, c->rec_far, c->fft_buf,
                    c->fft_tw, c->long_buf, c->d_rm, c->d_rm_lim, c->dsum, c->part, c->d_node_counts, c->flush_buf,
                    c->d_stage, c->d_time};
     for (void *p : dev)
@@ -181,6 +181,7 @@ static void release_buffers(ov_ctx *c)
     c->rec_out = c->rec_corr = c->rec_part = nullptr;
     c->rec_split = nullptr;
     c->rec_seg = nullptr;
+    c->rec_far = nullptr;
     c->fft_buf = c->fft_tw = nullptr;
     c->long_buf = nullptr;
     c->d_rm = nullptr;
@@ -193,7 +194,7 @@ static void release_buffers(ov_ctx *c)
     c->h_stage = c->h_corr = c->h_pf = c->h_pf_dev = c->h_time = nullptr;
     c->cap = c->n_live = 0;
     c->tcap = c->rm_cap = c->rm_lim_cap = c->pair_cap = c->loop_cap = c->loop_nodes_cap = 0;
-    c->rec_cap = c->rec_split_cap = c->rec_seg_cap = c->dsum_cap = 0;
+    c->rec_cap = c->rec_split_cap = c->rec_seg_cap = c->rec_far_cap = c->dsum_cap = 0;
     c->fft_cap = c->long_cap = c->loop_buf_cap = c->part_cap = c->rec_part_cap = c->h_corr_cap = 0;
     c->h_stage_bytes = c->d_stage_bytes = c->node_counts_cap = c->flush_bytes = 0;
     c->fft_M = 0;

@@ -274,7 +274,8 @@ struct ov_ctx {
     double *rec_out = nullptr, *rec_corr = nullptr, *rec_part = nullptr;
     float *rec_split = nullptr;
     CellFX *rec_seg = nullptr;       // fixed-point segments of the FP64 direct sums
-    int rec_seg_cap = 0;
+    float4 *rec_far = nullptr;       // segments of the candidates' far sums
+    int rec_seg_cap = 0, rec_far_cap = 0;
     double *h_corr = nullptr;    // pinned host copy of the corrections
     size_t h_corr_cap = 0;
     double *h_pf = nullptr;      // prefetched corrections (pinned, mapped host memory)

@@ -2380,6 +2380,299 @@ __global__ void __launch_bounds__(kRecThreads, 3) k_rec_sums(RecArgs r, const in
     if (threadIdx.x < kRecVals) out[threadIdx.x] = red[threadIdx.x][0];
 }
 
+// ------------------------------------------ candidates' sums, far segments
+//
+// The candidates' direct sums (k_rec_sums in mode 0) are 10^11 terms in a
+// reconnection pass of a large tangle.  For periodic images the 27 query
+// points are a grid (3 shifts an axis), and a segment s whose midpoint is at
+// least 8 |s| from every one of them has
+//     w = s-integral of R x s / |R|^3 = (R x s) / |R|^3 (1 + p(R.s / R^2, s^2 / R^2))
+// with R to the midpoint and p to fourth order (the next term is below
+// 0.063 / 8^6 = 2.4e-7).  So |R|^2 and R.s are sums of per-axis values, one
+// reciprocal square root serves the term, and the cross product is taken once
+// per segment: sum_j sc_j R_j has the components sum_i U_a[i] R_a[i], U_a[i]
+// the sc of the points with shift i on axis a.  About 17 FP32 operations and
+// one MUFU an interaction where the closed form takes 45 and three.  Two
+// candidates share a thread's segment in the two halves of the two-wide FP32
+// instructions.  Nearer segments, and those whose wrap is near its threshold,
+// take the closed form (FP64 near the query point) as k_rec_sums does.
+//
+// Error of a term relative to sc |R| |s| in units eps32: R 1, |R|^2 3, its
+// inverse root 4.5, the cube 15, the series 5, the sums U 9, the cross product
+// 4: below the 64 that k_rec_finish allows.
+
+// A segment for the series: A = (start's grid part, |s|), B = (midpoint less
+// that, squared distance from which the series holds), C = (s, s^2; 0: no
+// segment).
+struct FarSegment {
+    float4 A, B, C;
+};
+
+__device__ __forceinline__ FarSegment far_segment(const RecArgs &r, int m, int f)
+{
+    FarSegment o;
+    float ag[3], af[3], sv[3];
+    bool seg64 = false;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        ag[a] = r.sp[(size_t)a * r.cap + m];
+        af[a] = r.sp[(size_t)(3 + a) * r.cap + m];
+        float bg = r.sp[(size_t)a * r.cap + f], bf = r.sp[(size_t)(3 + a) * r.cap + f];
+        const float d = (bg - ag[a]) + (bf - af[a]);
+        if (r.geo.periodic[a]) {
+            // seg_pwrap: the end moved by a period toward the start
+            if (fabsf(fabsf(d) - r.hL[a]) < 1e-3f * r.hL[a] || fabsf(d) > 3.0f * r.hL[a]) seg64 = true;
+            if (d > r.hL[a]) { bg -= r.Lg[a]; bf -= r.Lf[a]; }
+            else if (d < -r.hL[a]) { bg += r.Lg[a]; bf += r.Lf[a]; }
+        }
+        sv[a] = (bg - ag[a]) + (bf - af[a]);
+    }
+    const float s2 = fmaf(sv[0], sv[0], fmaf(sv[1], sv[1], sv[2] * sv[2])), slen = sqrtf(s2);
+    const float near = sqrtf(r.rnear2) + 0.5f * slen;   // both ends beyond the FP64 radius
+    const float far2 = seg64 ? __int_as_float(0x7f800000) : fmaxf(64.0f * s2, near * near) * 1.0001f;
+    o.A = make_float4(ag[0], ag[1], ag[2], slen);
+    o.B = make_float4(fmaf(0.5f, sv[0], af[0]), fmaf(0.5f, sv[1], af[1]), fmaf(0.5f, sv[2], af[2]), far2);
+    o.C = make_float4(sv[0], sv[1], sv[2], seg64 && s2 == 0.0f ? 1e-30f : s2);
+    return o;
+}
+
+// Every segment's view for k_rec_far, three float4 arrays.
+__global__ void k_rec_segments(RecArgs r, float4 *__restrict__ seg)
+{
+    const int m = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m >= r.cap) return;
+    const int f = r.fwd[m];
+    FarSegment o;
+    o.A = o.B = o.C = make_float4(0, 0, 0, 0);
+    if (f >= 0 && f < r.cap) o = far_segment(r, m, f);
+    seg[m] = o.A;
+    seg[(size_t)r.cap + m] = o.B;
+    seg[2 * (size_t)r.cap + m] = o.C;
+}
+
+// Segment m -> f at candidate k by the closed form, every query point: t the
+// FP32 sum without kappa / 4 pi, t[3] its magnitude (sc |R| |s|), d the FP64
+// sum and its magnitude added.
+__device__ __noinline__ void rec_near(const RecArgs &r, int m, int f, int k, float t[4], double d[4])
+{
+    const double p[3] = {r.x[k], r.y[k], r.z[k]};
+    float ag[3], af[3], sv[3];
+    bool seg64 = false;
+    for (int a = 0; a < 3; ++a) {
+        ag[a] = r.sp[(size_t)a * r.cap + m];
+        af[a] = r.sp[(size_t)(3 + a) * r.cap + m];
+        float bg = r.sp[(size_t)a * r.cap + f], bf = r.sp[(size_t)(3 + a) * r.cap + f];
+        const float e = (bg - ag[a]) + (bf - af[a]);
+        if (r.geo.periodic[a]) {
+            if (fabsf(fabsf(e) - r.hL[a]) < 1e-3f * r.hL[a] || fabsf(e) > 3.0f * r.hL[a]) seg64 = true;
+            if (e > r.hL[a]) { bg -= r.Lg[a]; bf -= r.Lf[a]; }
+            else if (e < -r.hL[a]) { bg += r.Lg[a]; bf += r.Lf[a]; }
+        }
+        sv[a] = (bg - ag[a]) + (bf - af[a]);
+    }
+    const float slen = sqrtf(fmaf(sv[0], sv[0], fmaf(sv[1], sv[1], sv[2] * sv[2])));
+    float kg[3], kf[3];
+    for (int a = 0; a < 3; ++a) {
+        kg[a] = r.sp[(size_t)a * r.cap + k];
+        kf[a] = r.sp[(size_t)(3 + a) * r.cap + k];
+    }
+    for (int i = 0; i < 4; ++i) t[i] = 0.0f;
+    unsigned mask64 = 0;   // query points whose term is done in FP64
+#pragma unroll 3
+    for (int qi = (m == k || f == k) ? 1 : 0; qi <= r.geo.n_img; ++qi) {
+        const int j = qi - 1;
+        float R[3], P[3];
+        for (int a = 0; a < 3; ++a) {
+            float qg = kg[a], qf = kf[a];
+            if (j >= 0) { qg -= r.shift_g[j][a]; qf -= r.shift_f[j][a]; }
+            R[a] = (ag[a] - qg) + (af[a] - qf);
+            P[a] = R[a] + sv[a];
+        }
+        const float lR2 = fmaf(R[0], R[0], fmaf(R[1], R[1], R[2] * R[2]));
+        const float lp2 = fmaf(P[0], P[0], fmaf(P[1], P[1], P[2] * P[2]));
+        const float ra = rsqrtf(lR2), rb = rsqrtf(lp2), ab = ra * rb;
+        const float dot = fmaf(R[0], P[0], fmaf(R[1], P[1], R[2] * P[2])), nd = dot * ab;
+        const bool use64 = seg64 || !(fminf(lR2, lp2) >= r.rnear2) || fabsf(nd - 1e-8f) < 1e-4f;
+        if (use64) mask64 |= 1u << qi;
+        if (use64 || nd < 1e-8f) continue;   // (or the ndot filter, far from its threshold)
+        const float sc = __fdividef((ra + rb) * ab, fmaf(dot, ab, 1.0f));
+        t[0] = fmaf(fmaf(R[1], sv[2], -R[2] * sv[1]), sc, t[0]);
+        t[1] = fmaf(fmaf(R[2], sv[0], -R[0] * sv[2]), sc, t[1]);
+        t[2] = fmaf(fmaf(R[0], sv[1], -R[1] * sv[0]), sc, t[2]);
+        t[3] = fmaf(sc * slen, lR2 * ra, t[3]);
+    }
+    for (; mask64; mask64 &= mask64 - 1) {
+        double w[3];
+        if (rec_term64_fast(r, m, f, __ffs(mask64) - 2, p, w)) {
+            for (int a = 0; a < 3; ++a) d[a] += w[a];
+            d[3] += fabs(w[0]) + fabs(w[1]) + fabs(w[2]);
+        }
+    }
+}
+
+__device__ __forceinline__ float2 f2(float x) { return make_float2(x, x); }
+__device__ __forceinline__ float2 kahan_add2(float2 &s, float2 &c, float2 v)
+{
+    const float2 y = __fadd2_rn(v, make_float2(-c.x, -c.y));
+    const float2 t = __fadd2_rn(s, y);
+    const float2 e = __fadd2_rn(t, make_float2(-s.x, -s.y));
+    c = __fadd2_rn(e, make_float2(-y.x, -y.y));
+    s = t;
+    return s;
+}
+
+// The series for two (segment, query grid) combinations: R[a][i] the midpoint
+// from the query points with shift i - 1 on axis a, s the segment, s2 = s^2.
+// t: the sum of the terms without kappa / 4 pi; mg: sum of sc |R|; near2: a
+// bound from below on the smallest R^2 (the terms are void where the series
+// does not hold).  NZ: the image set is every shift in {-1, 0, 1}^3 with 1 to
+// NZ non-zero entries (periodic_26, _18, _6, open for 3 .. 0).
+template <int NZ>
+__device__ __forceinline__ void far_terms(const float2 R[3][3], const float2 s[3], float2 s2, float2 t[3], float2 &mg,
+                                          float2 &near2)
+{
+    float2 q2[3][3], qs[3][3], U[3][3];
+    near2 = f2(0);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            q2[a][i] = __fmul2_rn(R[a][i], R[a][i]);
+            qs[a][i] = __fmul2_rn(R[a][i], s[a]);
+            U[a][i] = f2(0);
+        }
+        near2.x += fminf(q2[a][1].x, fminf(q2[a][0].x, q2[a][2].x));
+        near2.y += fminf(q2[a][1].y, fminf(q2[a][0].y, q2[a][2].y));
+    }
+    mg = f2(0);
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            if ((i != 1) + (j != 1) > NZ) continue;
+            const float2 a2 = __fadd2_rn(q2[0][i], q2[1][j]), as = __fadd2_rn(qs[0][i], qs[1][j]);
+            float2 row = f2(0);
+#pragma unroll
+            for (int l = 0; l < 3; ++l) {
+                if ((i != 1) + (j != 1) + (l != 1) > NZ) continue;
+                const float2 R2 = __fadd2_rn(a2, q2[2][l]), Rs = __fadd2_rn(as, qs[2][l]);
+                float2 inv;
+                asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(inv.x) : "f"(R2.x));
+                asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(inv.y) : "f"(R2.y));
+                const float2 inv2 = __fmul2_rn(inv, inv);
+                const float2 x = __fmul2_rn(Rs, inv2), x2 = __fmul2_rn(x, x), y = __fmul2_rn(s2, inv2);
+                const float2 u = __ffma2_rn(f2(0.4921875f), x2, __ffma2_rn(f2(-0.328125f), y, f2(0.625f)));
+                const float2 v = __ffma2_rn(f2(0.0234375f), y, f2(-0.125f));
+                const float2 p = __ffma2_rn(x2, u, __ffma2_rn(y, v, f2(1.0f)));
+                const float2 sc = __fmul2_rn(__fmul2_rn(inv2, inv), p);
+                row = __fadd2_rn(row, sc);
+                U[2][l] = __fadd2_rn(U[2][l], sc);
+                mg = __fadd2_rn(mg, inv2);   // sc |R| = inv2 p, |p - 1| < 0.011
+            }
+            U[0][i] = __fadd2_rn(U[0][i], row);
+            U[1][j] = __fadd2_rn(U[1][j], row);
+        }
+    float2 V[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+        V[a] = __ffma2_rn(U[a][0], R[a][0], __ffma2_rn(U[a][1], R[a][1], __fmul2_rn(U[a][2], R[a][2])));
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const int b = (a + 1) % 3, c = (a + 2) % 3;
+        t[a] = __ffma2_rn(V[b], s[c], __fmul2_rn(V[c], make_float2(-s[b].x, -s[b].y)));
+    }
+    mg = __fmul2_rn(mg, f2(1.02f));
+}
+
+// Direct sums of the candidates.  Blocks: two candidates and a chunk of segments.
+template <int NZ>
+__global__ void __launch_bounds__(kRecThreads, 2) k_rec_far(const __grid_constant__ RecArgs r,
+                                                           const float4 *__restrict__ seg,
+                                                           const int *__restrict__ nodes, int n, int span,
+                                                           int max_chunks, double *__restrict__ part)
+{
+    __shared__ float2 s_q[3][3][2];   // axis, shift -1, 0, 1: minus the two query points' grid and fine parts
+    __shared__ double s_d[2][4][kRecThreads];   // FP64 sums and magnitudes
+    __shared__ double red[kRecVals][kRecThreads];
+    const int b0 = 2 * blockIdx.x, b1 = min(b0 + 1, n - 1), chunk = blockIdx.y;
+    const int k0 = nodes[b0], k1 = nodes[b1];
+    int lo, hi, lo1, hi1;
+    member_range(r, k0, lo, hi);
+    member_range(r, k1, lo1, hi1);
+    // candidates of two members: one after the other
+    const int turns = (lo == lo1 && hi == hi1) ? 1 : 2;
+    for (int turn = 0; turn < turns; ++turn) {
+        const int ka = turn ? k1 : k0, kb = turns == 1 ? k1 : ka;
+        if (turn) { lo = lo1; hi = hi1; }
+        const int m0 = lo + chunk * span, m1 = min(hi, m0 + span);
+        for (int e = 0; e < 2; ++e)
+            for (int v = 0; v < 4; ++v) s_d[e][v][threadIdx.x] = 0.0;
+        if (threadIdx.x < 18) {
+            const int e = threadIdx.x / 9, a = threadIdx.x % 9 / 3, i = threadIdx.x % 3, k = e ? kb : ka;
+            const float qg = r.sp[(size_t)a * r.cap + k], qf = r.sp[(size_t)(3 + a) * r.cap + k];
+            // the image at shift v is seen from p - L v
+            reinterpret_cast<float *>(&s_q[a][i][0])[e] = -(qg - (float)(i - 1) * r.Lg[a]);
+            reinterpret_cast<float *>(&s_q[a][i][1])[e] = -(qf - (float)(i - 1) * r.Lf[a]);
+        }
+        __syncthreads();
+        float2 s[3] = {f2(0), f2(0), f2(0)}, c[3] = {f2(0), f2(0), f2(0)}, mag = f2(0);
+        for (int m = m0 + threadIdx.x; m < m1; m += blockDim.x) {
+            const float4 A = __ldg(seg + m), B = __ldg(seg + (size_t)r.cap + m), C = __ldg(seg + 2 * (size_t)r.cap + m);
+            if (C.w == 0.0f) continue;
+            const float2 sv[3] = {f2(C.x), f2(C.y), f2(C.z)};
+            float2 R[3][3], t[3], mg, near2;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const float ga = a == 0 ? A.x : (a == 1 ? A.y : A.z), fa = a == 0 ? B.x : (a == 1 ? B.y : B.z);
+#pragma unroll
+                for (int i = 0; i < 3; ++i)
+                    R[a][i] = __fadd2_rn(__fadd2_rn(f2(ga), s_q[a][i][0]), __fadd2_rn(f2(fa), s_q[a][i][1]));
+            }
+            far_terms<NZ>(R, sv, f2(C.w), t, mg, near2);
+            mg = __fmul2_rn(mg, f2(A.w));
+            if (!(near2.x >= B.w && near2.y >= B.w)) {
+                for (int e = 0; e < 2; ++e) {
+                    if ((e ? near2.y : near2.x) >= B.w) continue;
+                    float nt[4];
+                    double nd[4] = {0, 0, 0, 0};
+                    rec_near(r, m, r.fwd[m], e ? kb : ka, nt, nd);
+                    for (int a = 0; a < 3; ++a) (e ? t[a].y : t[a].x) = nt[a];
+                    (e ? mg.y : mg.x) = nt[3];
+                    for (int v = 0; v < 4; ++v) s_d[e][v][threadIdx.x] += nd[v];
+                }
+            }
+            mag = __fadd2_rn(mag, mg);
+#pragma unroll
+            for (int a = 0; a < 3; ++a) kahan_add2(s[a], c[a], t[a]);
+        }
+        // the FP32 terms lack kappa / 4 pi (one more rounding: within the bound's 1.01)
+        const double f4 = r.f4pi;
+        for (int e = 0; e < 2; ++e) {
+            if (e && turns == 2) break;
+            const int b = turns == 1 ? (e ? b1 : b0) : (turn ? b1 : b0);
+            double abs1 = 0;
+            for (int a = 0; a < 3; ++a) {
+                const double v = e ? (double)s[a].y - (double)c[a].y : (double)s[a].x - (double)c[a].x;
+                red[a][threadIdx.x] = v * f4 + s_d[e][a][threadIdx.x];
+                abs1 += fabs((double)(e ? s[a].y : s[a].x));
+            }
+            red[3][threadIdx.x] = (double)(e ? mag.y : mag.x) * 1.0001 * f4;
+            red[4][threadIdx.x] = s_d[e][3][threadIdx.x];
+            red[5][threadIdx.x] = abs1 * f4;
+            red[6][threadIdx.x] = 0.0;
+            __syncthreads();
+            for (int off = blockDim.x / 2; off > 0; off >>= 1) {
+                if (threadIdx.x < off)
+                    for (int v = 0; v < kRecVals; ++v) red[v][threadIdx.x] += red[v][threadIdx.x + off];
+                __syncthreads();
+            }
+            if (threadIdx.x < kRecVals)
+                part[((size_t)b * max_chunks + chunk) * kRecVals + threadIdx.x] = red[threadIdx.x][0];
+            __syncthreads();
+        }
+    }
+}
+
 // The segments in fixed point for k_direct_fx: start, vector to the end moved
 // by a period toward it (seg_pwrap), zero where there is none.
 __global__ void k_segments_fx(RecArgs r, double fx_inv, CellFX *__restrict__ out)
@@ -2603,6 +2896,77 @@ __global__ void k_corr(RecArgs r, const int *__restrict__ cand, int c0, int nc, 
     for (int a = 0; a < 4; ++a) part[(size_t)idx * 4 + a] = out[a];
 }
 
+// k_corr and k_corr_finish for image sets that are grids of shifts: a warp takes
+// two candidates and a lane a changed segment, every query point at once by the
+// series of k_rec_far; the lanes' FP32 sums join by shuffles.
+template <int NZ>
+__global__ void __launch_bounds__(256, 2) k_corr_far(const __grid_constant__ RecArgs r, const int *__restrict__ cand,
+                                                     int c0, int nc, const __grid_constant__ RecChange ch,
+                                                     double *__restrict__ corr)
+{
+    const int lane = threadIdx.x & 31;
+    const int i0 = 2 * (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), i1 = min(i0 + 1, nc - 1);
+    if (i0 >= nc) return;
+    const int k[2] = {cand[c0 + i0], cand[c0 + i1]};
+    FarSegment S;
+    S.A = S.B = S.C = make_float4(0, 0, 0, 0);
+    const int m = lane < ch.n ? ch.m[lane] : -1, f = lane < ch.n ? ch.f[lane] : -1;
+    if (m >= 0 && m < r.cap && f >= 0 && f < r.cap) S = far_segment(r, m, f);
+    const bool live = S.C.w != 0.0f;   // else past the list, or no length
+    float2 R[3][3], t[3], mg, near2;
+    {
+        const float2 sv[3] = {f2(S.C.x), f2(S.C.y), f2(S.C.z)};
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const float ga = a == 0 ? S.A.x : (a == 1 ? S.A.y : S.A.z), fa = a == 0 ? S.B.x : (a == 1 ? S.B.y : S.B.z);
+            const size_t o = (size_t)a * r.cap, of = (size_t)(3 + a) * r.cap;
+#pragma unroll
+            for (int v = 0; v < 3; ++v) {
+                const float dg = (float)(v - 1) * r.Lg[a], df = (float)(v - 1) * r.Lf[a];
+                R[a][v] = __fadd2_rn(__fadd2_rn(f2(ga), make_float2(-(r.sp[o + k[0]] - dg), -(r.sp[o + k[1]] - dg))),
+                                     __fadd2_rn(f2(fa), make_float2(-(r.sp[of + k[0]] - df), -(r.sp[of + k[1]] - df))));
+            }
+        }
+        far_terms<NZ>(R, sv, f2(S.C.w), t, mg, near2);
+    }
+    const float sg = lane < ch.n ? (float)ch.sign[lane] : 0.0f;   // +-1
+#pragma unroll 1
+    for (int e = 0; e < 2; ++e) {
+        float w[4] = {e ? t[0].y : t[0].x, e ? t[1].y : t[1].x, e ? t[2].y : t[2].x, (e ? mg.y : mg.x) * S.A.w};
+        double acc[4] = {0, 0, 0, 0};
+        const bool near = live && !((e ? near2.y : near2.x) >= S.B.w);
+        if (near) rec_near(r, m, f, k[e], w, acc);
+        for (int a = 0; a < 4; ++a) w[a] = live ? (a < 3 ? sg * w[a] : w[a]) : 0.0f;
+        for (int a = 0; a < 3; ++a) acc[a] *= sg;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+            for (int a = 0; a < 4; ++a) w[a] += __shfl_xor_sync(0xffffffffu, w[a], o);
+        if (__any_sync(0xffffffffu, near)) {
+            for (int o = 16; o > 0; o >>= 1)
+                for (int a = 0; a < 4; ++a) acc[a] += __shfl_xor_sync(0xffffffffu, acc[a], o);
+        }
+        if (lane != 0 || (e && i1 == i0)) continue;
+        // 64 eps32 a term, 28 for its query points' sum (k_rec_finish), 5 for
+        // the lanes' additions
+        const double eps = 1.01 * 97.0 * 5.9604644775390625e-8;
+        double *cc = corr + 4 * (size_t)(c0 + (e ? i1 : i0));
+        double total = 0;
+        for (int a = 0; a < 3; ++a) {
+            const double d = fma((double)w[a], r.f4pi, acc[a]);
+            cc[a] += d;
+            total += fabs(d);
+        }
+        cc[3] += (eps * r.f4pi * (double)w[3] + 1e-12 * acc[3]) * (1.0 + 1e-9) + 1e-15 * total;
+    }
+}
+
+// The prefetched candidates' corrections into host memory.
+__global__ void k_corr_read(const double *__restrict__ corr, RecPrefetch pf, double *h_out)
+{
+    const int i = threadIdx.x >> 2, a = threadIdx.x & 3;
+    if (i < pf.n && i < kPrefetchMax) h_out[4 * i + a] = corr[4 * (size_t)pf.idx[i] + a];
+}
+
 // corr[4 c + {0,1,2}] += the query points' sums in order, corr[4 c + 3] +=
 // bound; then the prefetched candidates' corrections into host memory (h_out,
 // mapped: position i of the list at 4 i).
@@ -2692,6 +3056,24 @@ int rec_reserve(ov_ctx *c, int n, int max_chunks)
     return OV_OK;
 }
 
+// NZ of k_rec_far for the context's image set, -1 for any other set.
+int shift_grid(const Geometry &g)
+{
+    const int nz = g.n_img == 26 ? 3 : (g.n_img == 18 ? 2 : (g.n_img == 6 ? 1 : (g.n_img == 0 ? 0 : -1)));
+    unsigned seen = 0;
+    for (int j = 0; j < g.n_img && nz > 0; ++j) {
+        int id = 0, n = 0;
+        for (int a = 0; a < 3; ++a) {
+            if (g.shift[j][a] < -1 || g.shift[j][a] > 1) return -1;
+            id = 3 * id + g.shift[j][a] + 1;
+            n += g.shift[j][a] != 0;
+        }
+        if (g.nreflect[j] != 0 || n < 1 || n > nz || (seen >> id & 1)) return -1;
+        seen |= 1u << id;
+    }
+    return nz;
+}
+
 // FP64 sums of n nodes into rec_part: chunks of up to 8,192 segments, shorter
 // where few nodes would leave SMs without a block.
 int rec_launch_fx(ov_ctx *c, const RecArgs &ra, const int *d_nodes, int n, int *chunks)
@@ -2734,14 +3116,26 @@ int rec_launch_sums(ov_ctx *c, const int *d_nodes, int n, int mode, double *out_
     for (int j = 0; j < c->geo.n_img; ++j) mirror = mirror || c->geo.nreflect[j] > 0;
     if (mode == 1) {
         if ((r = rec_launch_fx(c, ra, d_nodes, n, &max_chunks))) return r;
+    } else if (mode == 0 && shift_grid(c->geo) >= 0) {
+        if (c->rec_far_cap < c->cap) {
+            if (c->rec_far) cudaFree(c->rec_far);
+            c->rec_far = nullptr;
+            c->rec_far_cap = 0;
+            OV_ALLOC(c, cudaMalloc(&c->rec_far, (size_t)c->cap * 3 * sizeof(float4)));
+            c->rec_far_cap = c->cap;
+        }
+        k_rec_segments<<<(c->cap + 255) / 256, 256, 0, c->stream>>>(ra, c->rec_far);
+        const int nz = shift_grid(c->geo);
+        auto *kernel = nz == 3 ? k_rec_far<3> : (nz == 2 ? k_rec_far<2> : (nz == 1 ? k_rec_far<1> : k_rec_far<0>));
+        kernel<<<dim3((n + 1) / 2, max_chunks), kRecThreads, 0, c->stream>>>(ra, c->rec_far, d_nodes, n, span,
+                                                                            max_chunks, c->rec_part);
+        c->launches++;
     } else if (mode == 2 && mirror)
         k_rec_sums<2, true><<<grid, kRecThreads, 0, c->stream>>>(ra, d_nodes, n, span, max_chunks, c->rec_part);
     else if (mode == 2)
         k_rec_sums<2, false><<<grid, kRecThreads, 0, c->stream>>>(ra, d_nodes, n, span, max_chunks, c->rec_part);
-    else if (mirror)
-        k_rec_sums<0, true><<<grid, kRecThreads, 0, c->stream>>>(ra, d_nodes, n, span, max_chunks, c->rec_part);
     else
-        k_rec_sums<0, false><<<grid, kRecThreads, 0, c->stream>>>(ra, d_nodes, n, span, max_chunks, c->rec_part);
+        k_rec_sums<0, true><<<grid, kRecThreads, 0, c->stream>>>(ra, d_nodes, n, span, max_chunks, c->rec_part);
     k_rec_finish<<<(n + 127) / 128, 128, 0, c->stream>>>(c->rec_part, n, max_chunks, c->rec_out);
     c->launches += 2;
     OV_CUDA(c, cudaGetLastError());
@@ -2852,7 +3246,16 @@ int ov_rec_correct(ov_ctx *c, int c0, int nc, const int *m, const int *f, const 
     list.n = npf;
     for (int i = 0; i < npf; ++i) list.idx[i] = pf[i];
     RecArgs ra = make_rec_args(c);
-    const int nq = c->geo.n_img + 1;
+    const int nq = c->geo.n_img + 1, nz = shift_grid(c->geo);
+    if (nz >= 0) {
+        auto *kernel = nz == 3 ? k_corr_far<3> : (nz == 2 ? k_corr_far<2> : (nz == 1 ? k_corr_far<1> : k_corr_far<0>));
+        kernel<<<((nc + 1) / 2 + 7) / 8, 256, 0, c->stream>>>(ra, c->rec_nodes, c0, nc, ch, c->rec_corr);
+        if (npf > 0) k_corr_read<<<1, 4 * kPrefetchMax, 0, c->stream>>>(c->rec_corr, list, c->h_pf_dev);
+        c->launches += npf > 0 ? 2 : 1;
+        OV_CUDA(c, cudaGetLastError());
+        OV_CUDA(c, cudaEventRecord(c->rec_ev, c->stream));
+        return OV_OK;
+    }
     k_corr<<<(nc * nq + 127) / 128, 128, 0, c->stream>>>(ra, c->rec_nodes, c0, nc, ch, c->rec_part);
     k_corr_finish<<<(nc + 127) / 128, 128, 0, c->stream>>>(c->rec_part, c0, nc, nq, c->rec_corr, list, c->h_pf_dev);
     c->launches += 2;
