@@ -215,8 +215,8 @@ typedef struct ov_tuning {
     int query_groups;
     int blocks_per_sm;
     int largest_first;
-    int high_occupancy;   /* mixed traversal variant: 0 the general kernel, 1 the same under a
-                             tighter register budget; 2, 3, 4 the periodic-image kernel with
+    int high_occupancy;   /* mixed traversal variant: 0 chosen by the node count, 1 the general
+                             kernel under a tighter register budget; 2, 3, 4 the periodic-image kernel with
                              fewer values held per lane (mirror images: as 0) with the
                              compiler's register count, 80 and 64 registers */
 } ov_tuning;

@@ -163,7 +163,7 @@ static void release_buffers(ov_ctx *c)
     ov_tree_free(c->tree);
     void *dev[] = {c->fwd, c->rev, c->status, c->pin, c->dnodes, c->d_tid, c->d_qorder, c->d_tprm, c->d_mrange,
                    c->d_pairs, c->d_npairs, c->d_loop_off, c->d_loop_nodes, c->d_loop_buf, c->d_loop_cut,
-                   c->rec_nodes, c->rec_pair, c->rec_out, c->rec_corr, c->rec_part, c->rec_split, c->rec_seg, c->rec_far, c->fft_buf,
+                   c->rec_nodes, c->rec_pair, c->rec_out, c->rec_corr, c->rec_part, c->rec_split, c->rec_seg, c->rec_far, c->near_lists, c->fft_buf,
                    c->fft_tw, c->long_buf, c->d_rm, c->d_rm_lim, c->dsum, c->part, c->d_node_counts, c->flush_buf,
                    c->d_stage, c->d_time};
     for (void *p : dev)
@@ -182,6 +182,8 @@ static void release_buffers(ov_ctx *c)
     c->rec_split = nullptr;
     c->rec_seg = nullptr;
     c->rec_far = nullptr;
+    c->near_lists = nullptr;
+    c->near_warps = 0;
     c->fft_buf = c->fft_tw = nullptr;
     c->long_buf = nullptr;
     c->d_rm = nullptr;
@@ -1129,8 +1131,8 @@ static unsigned long long graph_key(ov_ctx *c)
         h = mix64(h, lay, sizeof lay);
         h = mix64(h, &m.params, sizeof m.params);
     }
-    const void *ptrs[9] = {c->node.x, c->tree.cells, c->part, c->d_time, c->d_tid, c->d_tprm, c->d_qorder, c->d_mrange,
-                           c->tree.tt};
+    const void *ptrs[10] = {c->node.x, c->tree.cells, c->part, c->d_time, c->d_tid, c->d_tprm, c->d_qorder, c->d_mrange,
+                           c->tree.tt, c->near_lists};
     h = mix64(h, ptrs, sizeof ptrs);
     return h;
 }

@@ -274,6 +274,8 @@ struct ov_ctx {
     double *rec_out = nullptr, *rec_corr = nullptr, *rec_part = nullptr;
     float *rec_split = nullptr;
     CellFX *rec_seg = nullptr;       // fixed-point segments of the FP64 direct sums
+    int *near_lists = nullptr;       // the mixed traversals' deferred cells
+    size_t near_warps = 0;
     float4 *rec_far = nullptr;       // segments of the candidates' far sums
     int rec_seg_cap = 0, rec_far_cap = 0;
     double *h_corr = nullptr;    // pinned host copy of the corrections

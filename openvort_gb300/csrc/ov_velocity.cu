@@ -38,6 +38,7 @@ struct VelArgs {
     const DevParams *tprm;  // per-member parameters (null: prm)
     const int2 *mrange;     // per-member slot range [x, y) (null: [0, cap))
     int *work;              // work-queue counter
+    int *near_lists;        // mixed traversals: kNearCap * 32 deferred cells a warp of the grid
     int nt;                 // members
     int G;                  // query groups per node
     int S;                  // sub-walks per query point (FP64 split walk of a small tangle), else 1
@@ -288,18 +289,17 @@ __device__ __forceinline__ void image_point(const Geometry &g, int j, const doub
         const int f = g.reflect[j][m];
         if (f < 0 || f > 5) continue;
         // (selected, not indexed: the arrays stay in registers)
-#pragma unroll
-        for (int ax = 0; ax < 3; ++ax)
-            if (f >> 1 == ax) q[ax] = rn_sub(rn_mul(2.0, (f & 1) ? g.hi[ax] : g.lo[ax]), p[ax]);
+        int ax = f >> 1;
+        double w = (f & 1) ? g.hi[ax] : g.lo[ax];
+        q[ax] = rn_sub(rn_mul(2.0, w), p[ax]);
     }
 }
 
 __device__ __forceinline__ void mirror_vec(int f, double v[3])
 {
     // mirror_vector_reflect (boundaries.c:201-211): normal component flips
-#pragma unroll
-    for (int ax = 0; ax < 3; ++ax)
-        if (f >> 1 == ax) v[ax] = -v[ax];
+    int ax = f >> 1;
+    v[ax] = -v[ax];
 }
 
 // The segment law (octree.c:321-342 / tangle.c:536-559) for R = COM - r
@@ -819,7 +819,15 @@ __device__ __forceinline__ void kahan_add(float &s, float &c, float v)
     s = t;
 }
 
-constexpr int kNearCap = 24;   // deferred near-field leaves per lane
+// Deferred near-field leaves per lane.  The lists are in global memory, a few
+// coalesced words a walk: in shared memory they would take the L1 that the walk's
+// cells need, and be too short for dense tangles, whose overflow is evaluated in
+// FP64 inside the walk (262,144 nodes: 5.8 ms with 24 entries, 5.1 with 96;
+// 1,048,576: 44.5 ms with 24 in shared memory, 20.4 now).
+constexpr int kNearCap = 96;
+// The spherical section has a warp for each tile and query point, not a grid that
+// stays: lists in shared memory, which need no room per warp of the launch.
+constexpr int kNearCapSph = 24;
 // d^2 below Cell32::thr times this opens a cell clear of the guard band
 constexpr float kThrLo = (1.0f - 2e-5f) / (1.0f + 2e-5f);
 
@@ -929,10 +937,11 @@ struct MixedAcc {
 // One query point (g + f split, image j; j < 0 the node itself) for the 32
 // lanes of a warp.  Near-field leaves are appended to the lane's list
 // (cell, image) and evaluated in FP64 after all query points.
+template <int Cap>
 __device__ __forceinline__ void bh_query32(const VelArgs &a, const float g[3], const float f[3], const double p[3],
                                            int j, bool part, int root, int ncell, MixedAcc &m, int *near_list,
                                            int &nnear, double w64[3], bool &overflow)
-// near_list: this lane's column of a shared [kNearCap][32] array, stride 32.
+// near_list: this lane's column of a [Cap][32] array, stride 32.
 {
     const float near2 = a.near2f;
     const float f4pi = a.f4pif;
@@ -995,7 +1004,7 @@ __device__ __forceinline__ void bh_query32(const VelArgs &a, const float g[3], c
                 if (defer) {
                     // near field, or a filter inside its guard band: FP64, after the traversal
                     ++m.nnear;
-                    if (nnear < kNearCap) {
+                    if (nnear < Cap) {
                         near_list[32 * nnear] = (c << 5) | (j + 1);
                         ++nnear;
                     } else {
@@ -1044,8 +1053,7 @@ __global__ void __launch_bounds__(32 * W, (min_blocks_mixed<W, HI>())) k_vel_mix
     const int lane = threadIdx.x & 31;
     const int tiles = a.counters[TC_ITEMS];
     const int items = tiles * a.G;
-    __shared__ int s_near[W][kNearCap * 32];   // per warp: [entry][lane]
-    int *near_list = &s_near[threadIdx.x >> 5][lane];
+    int *near_list = a.near_lists + ((size_t)blockIdx.x * W + (threadIdx.x >> 5)) * (kNearCap * 32) + lane;   // [entry][lane]
     unsigned visits = 0, accepts = 0, steps = 0, fallback = 0, near64 = 0;   // per lane
     bool overflow = false;
     for (int it = next_item(a); it < items; it = next_item(a)) {
@@ -1094,7 +1102,7 @@ __global__ void __launch_bounds__(32 * W, (min_blocks_mixed<W, HI>())) k_vel_mix
                 }
                 MixedAcc mr = {0, 0, 0, 0, 0, 0, 0u, 0u, 0u, 0u, 0u};
                 double wr[3] = {0, 0, 0};   // FP64 terms of this image when the near list is full
-                bh_query32(a, g, f, p, j, part, w.root, w.end, mr, near_list, nnear, wr, overflow);
+                bh_query32<kNearCap>(a, g, f, p, j, part, w.root, w.end, mr, near_list, nnear, wr, overflow);
                 double v[3] = {acc_value(mr.s0, mr.c0) + wr[0], acc_value(mr.s1, mr.c1) + wr[1],
                                acc_value(mr.s2, mr.c2) + wr[2]};
                 for (int r = 0; r < a.geo.nreflect[j]; ++r) mirror_vec(a.geo.reflect[j][r], v);
@@ -1102,7 +1110,7 @@ __global__ void __launch_bounds__(32 * W, (min_blocks_mixed<W, HI>())) k_vel_mix
                 m.nvis += mr.nvis; m.nacc += mr.nacc; m.nstep += mr.nstep; m.nfb += mr.nfb; m.nnear += mr.nnear;
                 continue;
             }
-            bh_query32(a, g, f, p, j, part, w.root, w.end, m, near_list, nnear, w64, overflow);
+            bh_query32<kNearCap>(a, g, f, p, j, part, w.root, w.end, m, near_list, nnear, w64, overflow);
         }
         // deferred near-field interactions, all lanes together
         for (int i = 0; i < nnear && i < kNearCap; ++i) {
@@ -1161,7 +1169,7 @@ __global__ void __launch_bounds__(32 * W, (min_blocks_mixed<W, HI>())) k_vel_mix
 // paths instead of kept, those paths out of line, and the circulation of a
 // cell read only when some lane accepts it.  Same decisions, arithmetic and
 // summation order as k_vel_mixed; the register budget is a template
-// parameter (more resident warps against spills), picked by the autotuner.
+// parameter (more resident warps against spills).
 
 // (the rare paths are kept out of line: their FP64 temporaries would
 // otherwise raise the register count of the walk loop)
@@ -1302,8 +1310,7 @@ __global__ void __launch_bounds__(32 * W, (min_blocks_mixp<W, R>())) k_vel_mixp(
     const int lane = threadIdx.x & 31;
     const int tiles = a.counters[TC_ITEMS];
     const int items = tiles * a.G;
-    __shared__ int s_near[W][kNearCap * 32];   // per warp: [entry][lane]
-    int *near_list = &s_near[threadIdx.x >> 5][lane];
+    int *near_list = a.near_lists + ((size_t)blockIdx.x * W + (threadIdx.x >> 5)) * (kNearCap * 32) + lane;   // [entry][lane]
     unsigned visits = 0, accepts = 0, steps = 0, fallback = 0, near64 = 0;   // per lane
     bool overflow = false;
     for (int it = next_item(a); it < items; it = next_item(a)) {
@@ -1732,10 +1739,11 @@ __global__ void __launch_bounds__(32 * W, min_blocks_split<W>()) k_vel_split(Vel
 
 }  // namespace
 
-// Query groups per node: the tuned value, else enough warps for ~32 per SM
-// on small tangles (~400 for the FP64 split walk, whose work items are
-// longer: finer items balance the end of the launch.  65,536 nodes: 4.1 ms
-// with 8 groups, 3.9 with 14, 3.7 with 27).
+// Query groups per node: the tuned value, else enough warps for ~32 per SM on
+// small tangles, ~400 for the split walk: its work items are longer, and finer
+// ones balance the end of the launch (65,536 nodes: 4.1 ms with 8 groups, 3.9
+// with 14, 3.7 with 27).  The mixed traversal's FP32 sums depend on the groups
+// in the last digits of their 1e-8.
 int ov_query_groups(ov_ctx *c)
 {
     int maxg = c->geo.n_img + 1;
@@ -1832,6 +1840,48 @@ static int ov_sub_walks(const ov_ctx *c, int precision)
     return ov_split_walk(c, precision) ? sub_walks_for(c->cap) : 1;
 }
 
+static bool has_mirror_images(const Geometry &g)
+{
+    for (int j = 0; j < g.n_img; ++j)
+        if (g.nreflect[j] > 0) return true;
+    return false;
+}
+
+// variant (Tuning::hi_occ) of the mixed traversal: 1 k_vel_mixed under a
+// tighter register budget, 2-4 k_vel_mixp (periodic image sets only) with the
+// compiler's register count, 80 and 64 registers.  0 picks one, all give the
+// same sums: with at least 48 work items an SM the walk's latency is best hidden by
+// 32 warps (k_vel_mixp at 64 registers, against k_vel_mixed: 262,144 nodes 5.15
+// against 5.5 ms, 1,048,576 20.4 against 24.0); with fewer their tiles lie too far
+// apart to share cells (32,768 nodes 1.24 against 1.00, 65,536 1.57 against 1.30).
+// Few long items (all 27 query points, or half of them) finish earlier on 24
+// warps than on 20 (114,688 nodes 2.10 against 2.45).  Mirror images: k_vel_mixed.
+constexpr int kMixpItems = 48, kFewItems = 40;
+static int mixed_variant(ov_ctx *c)
+{
+    if (c->tune.hi_occ || has_mirror_images(c->geo)) return c->tune.hi_occ;
+    long long tiles = 0;
+    for (const Member &m : c->mem) tiles += (m.n + 31) / 32;
+    const int G = ov_query_groups(c);
+    const long long items = tiles * G / c->sm_count;
+    if (items >= kMixpItems) return 4;
+    return G == 1 || (G == 2 && items >= kFewItems) ? 1 : 0;
+}
+
+static int launch_warps(const ov_ctx *c) { return c->tune.warps == 2 || c->tune.warps == 8 ? c->tune.warps : 4; }
+
+// Room for the deferred lists of `warps` warps (mixed traversals).
+static int reserve_near_lists(ov_ctx *c, size_t warps)
+{
+    if (c->near_warps >= warps) return OV_OK;
+    if (c->near_lists) cudaFree(c->near_lists);
+    c->near_lists = nullptr;
+    c->near_warps = 0;
+    OV_ALLOC(c, cudaMalloc(&c->near_lists, warps * kNearCap * 32 * sizeof(int)));
+    c->near_warps = warps;
+    return OV_OK;
+}
+
 int ov_reserve_velocity_scratch(ov_ctx *c)
 {
     int G = ov_query_groups(c);
@@ -1842,21 +1892,15 @@ int ov_reserve_velocity_scratch(ov_ctx *c)
         OV_ALLOC(c, cudaMalloc(&c->part, need * sizeof(double)));
         c->part_cap = need;
     }
+    if (c->precision == OV_PREC_MIXED) {
+        const int warps = launch_warps(c), r = reserve_near_lists(c, (size_t)ov_traversal_blocks(c, c->precision, warps, nullptr) * warps);
+        if (r) return r;
+    }
     return OV_OK;
 }
 
 // Traversal kernel for a precision and block shape.
 typedef void (*VelKernel)(VelArgs, double *);
-static bool has_mirror_images(const Geometry &g)
-{
-    for (int j = 0; j < g.n_img; ++j)
-        if (g.nreflect[j] > 0) return true;
-    return false;
-}
-
-// variant (Tuning::hi_occ) of the mixed traversal: 0 k_vel_mixed, 1 the
-// same under a tighter register budget, 2-4 k_vel_mixp (periodic image sets
-// only) with the compiler's register count, 80 and 64 registers
 template <int R> static VelKernel mixp_kernel(int warps)
 {
     if (warps == 2) return k_vel_mixp<2, R>;
@@ -1902,7 +1946,7 @@ static size_t list_bytes(const ov_ctx *c, int precision, int warps)
 // every SM, but no more blocks than there can be work items.
 int ov_traversal_blocks(ov_ctx *c, int precision, int warps, int *per_sm)
 {
-    VelKernel k = vel_kernel(precision, ov_split_walk(c, precision), warps, c->tune.hi_occ, has_mirror_images(c->geo));
+    VelKernel k = vel_kernel(precision, ov_split_walk(c, precision), warps, mixed_variant(c), has_mirror_images(c->geo));
     int occ = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, 32 * warps, list_bytes(c, precision, warps)) !=
             cudaSuccess || occ < 1) {
@@ -1927,8 +1971,7 @@ int ov_launch_velocities(ov_ctx *c, const NodeArrays &na, double t, int precisio
     }
     int r = ov_reserve_velocity_scratch(c);
     if (r) return r;
-    int warps = c->tune.warps;
-    if (warps != 2 && warps != 8) warps = 4;
+    const int warps = launch_warps(c);
     int blocks = ov_traversal_blocks(c, precision, warps, nullptr);
     if (c->count_nodes && c->time_dev_index < 0) {
         // per-target counters (not inside the captured RK4 graph)
@@ -1943,8 +1986,13 @@ int ov_launch_velocities(ov_ctx *c, const NodeArrays &na, double t, int precisio
         OV_CUDA(c, cudaMemsetAsync(c->d_node_counts, 0, need * sizeof(unsigned), s));
         a.node_counts = c->d_node_counts;
     }
+    a.near_lists = nullptr;
+    if (precision == OV_PREC_MIXED) {
+        if ((r = reserve_near_lists(c, (size_t)blocks * warps))) return r;
+        a.near_lists = c->near_lists;
+    }
     OV_CUDA(c, cudaMemsetAsync(a.work, 0, sizeof(int), s));
-    vel_kernel(precision, ov_split_walk(c, precision), warps, c->tune.hi_occ, has_mirror_images(c->geo))<<<
+    vel_kernel(precision, ov_split_walk(c, precision), warps, mixed_variant(c), has_mirror_images(c->geo))<<<
         blocks, 32 * warps, list_bytes(c, precision, warps), s>>>(a, c->part);
     if (a.S > 1) {
         const long long threads = 6LL * c->cap * a.G;
@@ -3686,7 +3734,7 @@ __global__ void __launch_bounds__(128) k_sph_query(SphArgs s, double *__restrict
 __global__ void __launch_bounds__(128) k_sph_query_mixed(SphArgs s, double *__restrict__ part)
 {
     const VelArgs &a = s.v;
-    __shared__ int s_near[4][kNearCap * 32];
+    __shared__ int s_near[4][kNearCapSph * 32];
     const int lane = threadIdx.x & 31;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     int *near_list = &s_near[threadIdx.x >> 5][lane];
@@ -3723,8 +3771,8 @@ __global__ void __launch_bounds__(128) k_sph_query_mixed(SphArgs s, double *__re
     double w64[3] = {0, 0, 0};
     int nnear = 0;
     bool overflow = false;
-    bh_query32(a, g, f, qp, -1, go, root, end, acc, near_list, nnear, w64, overflow);
-    for (int i = 0; i < nnear && i < kNearCap; ++i) {
+    bh_query32<kNearCapSph>(a, g, f, qp, -1, go, root, end, acc, near_list, nnear, w64, overflow);
+    for (int i = 0; i < nnear && i < kNearCapSph; ++i) {
         const int e = near_list[32 * i];
         const int c = e >> 5;
         if (c < root || c >= end) { bad_index(a, 3, e); continue; }

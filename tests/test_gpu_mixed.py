@@ -102,3 +102,34 @@ def test_mixed_kernel_variants_agree():
     for ho, warps, acc, vis, v in out[1:]:
         assert acc == acc0 and vis == vis0, (ho, warps)
         np.testing.assert_array_equal(v, v0, err_msg=f"variant {ho}, {warps} warps")
+
+
+@pytest.mark.parametrize("loops,per_loop,D,images,groups", [
+    (2, 33, 0.1, None, 0),              # two tiles and a remainder of two nodes
+    (450, 256, 0.1, None, 0),           # two query groups, long items
+    (950, 256, 0.1, None, 0),           # one query group
+    (24, 512, 0.002, None, 1),          # dense: more than 96 deferred cells a lane
+    (24, 512, 0.002, "wall_1_26", 1),   # the same with mirror images
+])
+def test_mixed_automatic_variant_agrees(loops, per_loop, D, images, groups):
+    """The variant that is picked by the node count gives the sums of the general
+    kernel bit for bit, with full deferred lists too."""
+    ht = W.random_walk_tangle(loops, per_loop, D=D, seed=4)
+    if images:
+        ht = W.HostTangle(ht.pos.copy(), ht.conn[:, 0].copy(), ht.conn[:, 1].copy(), ht.box_lo, ht.box_hi,
+                          image_set=images)
+    ctx = gpu.Context(0, params=W.config_params("rw"), precision=abi.OV_PREC_MIXED)
+    ctx.upload(ht)
+    out = []
+    for ho in (0, 1, 2):
+        ctx.set_tuning(query_groups=groups, high_occupancy=ho)
+        ctx.update_tangle(0.0)
+        st = ctx.stats()
+        assert st["error_word"] == 0
+        if groups == 1:
+            assert st["near_field_fp64"] > 96 * loops * per_loop   # some lane's list was full
+        out.append((st["accepts"], st["visits"], np.array(ctx.download(ht, abi.OV_F_VELS).vels)))
+    ctx.close()
+    for acc, vis, v in out[1:]:
+        assert acc == out[0][0] and vis == out[0][1]
+        np.testing.assert_array_equal(v, out[0][2])
