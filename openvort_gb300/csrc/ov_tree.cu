@@ -491,21 +491,6 @@ __device__ __forceinline__ void store_psum(double *psum, int ci, const double ac
     psum[3 * (size_t)ci + 2] = acc[2];
 }
 
-// Add a finished cell's sums to acc (position sum, circulation sum), in
-// the order of a sum over its children: a one-node cell's mean is its
-// position (a product with 1.0), larger cells keep the sum in psum.
-__device__ __forceinline__ void add_cell_sums(const Cell64 &c, const double *psum, int ci, double acc[6])
-{
-    double p0 = c.cx, p1 = c.cy, p2 = c.cz;
-    if (c.count != 1) {
-        p0 = psum[3 * (size_t)ci];
-        p1 = psum[3 * (size_t)ci + 1];
-        p2 = psum[3 * (size_t)ci + 2];
-    }
-    acc[0] = rn_add(acc[0], p0); acc[1] = rn_add(acc[1], p1); acc[2] = rn_add(acc[2], p2);
-    acc[3] = rn_add(acc[3], c.qx); acc[4] = rn_add(acc[4], c.qy); acc[5] = rn_add(acc[5], c.qz);
-}
-
 // A node's moment as k_keys stored it (6 doubles at 48-byte stride).
 __device__ __forceinline__ void load_moment(const double *nm, int id, double m[6])
 {
@@ -682,6 +667,10 @@ __global__ void k_cells(const uint64_t *__restrict__ keys, const int *__restrict
 
 // Above this many slots the level sums run as one launch per level.
 constexpr int kLevelLaunchSlots = 1 << 19;
+// Threads of a k_levels block: a small tree stays in one block, whose levels
+// need no grid barrier (256, 512, 1024 threads: tree of 496 nodes 0.155, 0.141,
+// 0.135 ms, of 4,125 nodes 0.171, 0.163, 0.169).
+constexpr int kLevelThreads = 512;
 
 // Grid-wide barrier of the cooperative k_levels (all blocks resident): one
 // arrival per block on a counter cleared by the build, then a bounded wait
@@ -692,6 +681,7 @@ constexpr unsigned kBarrierSpins = 1u << 22;   // of at least 64 ns each
 __device__ __forceinline__ bool grid_barrier(unsigned *count, unsigned epoch, int *counters)
 {
     __syncthreads();
+    if (gridDim.x == 1) return true;
     int ok = 1;
     if (threadIdx.x == 0) {
         __threadfence();   // this block's sums before the arrival
@@ -753,6 +743,80 @@ __device__ __forceinline__ void level_cell(int ci, int lev, int ncell, int *coun
     store_cell(cells, ci, acc, cnt, lm, lev, ch, views);
 }
 
+// The same with eight lanes to a cell (whole warps; lane k = lane & 7 of a
+// group): lane k < 6 adds component k of the children's sums and finishes it,
+// in level_cell's order and roundings.  An FP64 instruction holds the warp's
+// scheduler for 70 cycles however many lanes it serves, and one thread a cell
+// issues six to a child: fewer cells to the instruction, but a chain a quarter
+// as long, where the levels are too small to fill the GPU.
+struct LaneSum {
+    double acc;      // lane k < 6: component k
+    int next, cnt;   // successor, nodes
+    bool ok;
+};
+__device__ __forceinline__ LaneSum lane_children(bool go, int k, int ch, int lev, int end, const Cell64 *cells,
+                                                 const uint8_t *lvl8, const double *psum)
+{
+    LaneSum r = {0.0, ch, 0, true};
+    const bool all = go;
+    int nc = 0;
+    while (__any_sync(0xffffffffu, go)) {
+        if (!go) continue;
+        const int lv = __ldcg(&lvl8[r.next]);
+        const int2 nx = __ldcg(reinterpret_cast<const int2 *>(cells + r.next) + 7);   // successor, count
+        double v = 0, ps = 0;
+        if (k < 6) v = __ldcg(reinterpret_cast<const double *>(cells + r.next) + k);
+        if (k < 3) ps = __ldcg(&psum[3 * (size_t)r.next + k]);
+        if (lv != lev || nc == 8) { go = false; r.ok = nc > 0 && lv != lev; continue; }
+        r.acc = rn_add(r.acc, k < 3 && nx.y != 1 ? ps : v);
+        r.cnt += nx.y;
+        ++nc;
+        if (nx.x <= r.next) { go = false; r.ok = false; continue; }
+        r.next = nx.x;
+        go = r.next < end;
+    }
+    r.ok = r.ok || !all;
+    return r;
+}
+
+// store_cell by the eight lanes of a group (Lm is in the cell; `ok` is the
+// group's): count > 1 or one node whose sum is its mean.
+__device__ __forceinline__ void lane_store(bool ok, int k, int ci, const LaneSum &r, float thr, float lm32,
+                                           Cell64 *cells, const CellViews &v)
+{
+    double c = r.acc;
+    if (r.cnt != 1 && k < 3) c = rn_mul(c, r.cnt < TREE_INV_COUNT ? v.inv_count[r.cnt] : 1.0 / (double)r.cnt);
+    if (ok && k < 6) reinterpret_cast<double *>(cells + ci)[k] = c;
+    if (ok && k == 7) reinterpret_cast<int2 *>(cells + ci)[7] = make_int2(r.next, r.cnt);
+    if (v.c32) {
+        float *o = reinterpret_cast<float *>(v.c32 + ci);
+        const double G = k < 3 ? rint(c * v.inv_h) * v.h : 0.0;
+        const float hi = k < 3 ? (float)G : (float)c;
+        if (ok && k < 3) { o[k] = hi; o[4 + k] = (float)(c - G); }
+        else if (ok && k < 6) o[8 + k - 3] = hi;
+        else if (ok && k == 6) { o[3] = thr; o[7] = __int_as_float(r.next); o[11] = lm32; }
+    }
+    if (v.cfx) {
+        const bool in = k >= 6 || fabs(c * v.fx_inv) < kFxLimit;
+        const int64_t w = __double2ll_rn(c * v.fx_inv);
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        const int g8 = threadIdx.x & 24;
+        int64_t x[3], q[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            x[a] = __shfl_sync(0xffffffffu, w, g8 + a);
+            q[a] = __shfl_sync(0xffffffffu, w, g8 + 3 + a);
+        }
+        if (ok && k == 0) {
+            const CellFX o = fx_cell(x, q, ((m >> g8) & 63u) == 63u);
+            const int4 *src = reinterpret_cast<const int4 *>(&o);
+            int4 *dst = reinterpret_cast<int4 *>(v.cfx + ci);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) dst[i] = src[i];
+        }
+    }
+}
+
 // One level of the bottom-up sums per launch (large trees: the levels hold
 // enough cells to fill the GPU, and launches cost less than grid barriers).
 __global__ void k_level(int lev, const int *__restrict__ lvl_cnt, const int *__restrict__ lvl_list,
@@ -775,6 +839,9 @@ __global__ void k_level(int lev, const int *__restrict__ lvl_cnt, const int *__r
 // cooperative launch (small trees, where a launch per level would cost more
 // than the level's work): the blocks share each level's list, then meet at a
 // grid barrier (levels without cells are skipped by every block alike).
+// Eight lanes to a cell and blocks enough to give every SM a part of the widest
+// level: 128 us at 65,536 nodes with a thread a cell on 64 blocks, 97 now; what
+// remains is a level's chain (list, children one after the other, store, barrier).
 // The leaves were finished by k_cells.
 __global__ void k_levels(int lev_hi, const int *__restrict__ lvl_cnt, const int *__restrict__ lvl_list,
                          unsigned *barrier, const int *__restrict__ cell_off, int *counters, int cap_cells,
@@ -790,9 +857,19 @@ __global__ void k_levels(int lev_hi, const int *__restrict__ lvl_cnt, const int 
         const int n = lvl_cnt[lev];
         start -= n;   // level lev's list is [start, start + n)
         if (n == 0) continue;
-        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-            const int ci = start + i < cap_cells ? lvl_list[start + i] : -1;
-            level_cell(ci, lev, ncell, counters, cells, lvl8, psum, views);
+        for (int i0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5 << 2; i0 < n; i0 += gridDim.x * blockDim.x >> 3) {
+            const int i = i0 + ((threadIdx.x & 31) >> 3), k = threadIdx.x & 7;
+            const bool mine = i < n;
+            int ci = mine && start + i < cap_cells ? lvl_list[start + i] : 0;
+            bool ok = mine && ci > 0 && ci < ncell - 1;
+            if (!ok) ci = 0;
+            const double lm = !views.lev_tab && k == 6 && ok ? cells[ci].lm : 0.0;
+            const LaneSum r = lane_children(ok, k, ci + 1, lev + 1, ncell, cells, lvl8, psum);
+            ok = ok && r.ok;
+            if (mine && !ok) atomicOr(&counters[TC_ERR], OV_EW_BOUNDS);
+            if (ok && k < 3) psum[3 * (size_t)ci + k] = r.acc;
+            lane_store(ok, k, ci, r, views.lev_tab ? views.lev_tab[lev] : cell_thr(lm, views.theta),
+                       views.lev_tab ? views.lev_tab[TREE_LV_SLOTS + lev] : __double2float_ru(lm), cells, views);
         }
         if (lev > 1 && !grid_barrier(barrier, epoch++, counters)) return;
     }
@@ -801,8 +878,9 @@ __global__ void k_levels(int lev_hi, const int *__restrict__ lvl_cnt, const int 
 // Roots, one block per member: level-1 children plus the nodes outside the
 // root box; also the one-node and empty members.
 __global__ void k_root(const int *__restrict__ order, const int *__restrict__ cell_off, int *counters,
-                       int *tt, const double *__restrict__ nm, KeyGeom g, Cell64 *cells, const double *psum,
-                       int *first, int cap_cells, CellViews views)
+                       int *tt, const double *__restrict__ nm, KeyGeom g, Cell64 *cells,
+                       const uint8_t *__restrict__ lvl8, const double *psum, int *first, int cap_cells,
+                       CellViews views)
 {
     __shared__ double red[6][256];
     int *w = tt + blockIdx.x * TT_WORDS;
@@ -825,34 +903,28 @@ __global__ void k_root(const int *__restrict__ order, const int *__restrict__ ce
     if (nne == 1 && M == 1 && threadIdx.x == 0) load_moment(nm, order[st], acc);
     for (int k = 0; k < 6; ++k) red[k][threadIdx.x] = acc[k];
     __syncthreads();
-    for (int off = blockDim.x / 2; off > 0; off >>= 1) {
+    // (few nodes outside: the steps that would only add zeros are left out)
+    int off = blockDim.x / 2;
+    while (off > 0 && off >= nout) off >>= 1;
+    for (; off > 0; off >>= 1) {
         if (threadIdx.x < off)
             for (int k = 0; k < 6; ++k) red[k][threadIdx.x] = rn_add(red[k][threadIdx.x], red[k][threadIdx.x + off]);
         __syncthreads();
     }
-    if (threadIdx.x != 0) return;
-    double sum[6];
-    for (int k = 0; k < 6; ++k) sum[k] = 0;
-    if (nne >= 2) {
-        for (int ch = root + 1; ch < end && ch > root; ch = cells[ch].next)
-            add_cell_sums(cells[ch], psum, ch, sum);
-    }
-    for (int k = 0; k < 6; ++k) sum[k] = rn_add(sum[k], red[k][0]);
-    Cell64 r;
-    double inv = 1.0 / (double)nne;
-    r.cx = rn_mul(sum[0], inv); r.cy = rn_mul(sum[1], inv); r.cz = rn_mul(sum[2], inv);
-    r.qx = sum[3]; r.qy = sum[4]; r.qz = sum[5];
-    const int mem = blockIdx.x < OV_SPH_MEMBERS ? blockIdx.x : 0;
-    r.lm = g.sph_root ? sph_box_lm(g.sb[mem], g.st[mem]) : box_lm(g.lo, g.hi);
+    if (threadIdx.x >= 32) return;
+    // the first eight lanes finish the root: 16.1 us a launch with one thread, 12.7 so,
+    // for 496 and 65,536 nodes
+    const int k = threadIdx.x & 7, lane = threadIdx.x;
+    LaneSum r = lane_children(lane < 8 && nne >= 2 && end > root + 1, k, root + 1, 1, end, cells, lvl8, psum);
+    if (lane == 0 && !r.ok) atomicOr(&counters[TC_ERR], OV_EW_BOUNDS);
+    if (k < 6) r.acc = rn_add(r.acc, red[k][0]);
     r.next = end;
-    r.count = nne;
-    cells[root] = r;
-    first[root] = st;
-    const double c[3] = {r.cx, r.cy, r.cz}, q[3] = {r.qx, r.qy, r.qz};
-    if (views.c32)
-        write_cell32(views.c32, root, c, q, cell_thr(r.lm, views.theta), __double2float_ru(r.lm), r.next, views.h,
-                     views.inv_h);
-    if (views.cfx) write_cellfx(views.cfx, root, c, q, views.fx_inv);
+    r.cnt = nne;
+    const int mem = blockIdx.x < OV_SPH_MEMBERS ? blockIdx.x : 0;
+    const double lm = g.sph_root ? sph_box_lm(g.sb[mem], g.st[mem]) : box_lm(g.lo, g.hi);
+    if (lane == 6) cells[root].lm = lm;
+    if (lane == 7) first[root] = st;
+    lane_store(lane < 8, k, root, r, cell_thr(lm, views.theta), __double2float_ru(lm), cells, views);
 }
 
 }  // namespace
@@ -1017,18 +1089,18 @@ int ov_tree_build(ov_ctx *c, const NodeArrays &na, cudaStream_t s)
         // the level sums: one cooperative launch, every block resident
         static int per_sm = 0;
         if (!per_sm) {
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_levels, 256, 0);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_levels, kLevelThreads, 0);
             per_sm = per_sm > 0 ? per_sm : 1;
         }
-        const int want = std::max(1, cap / 1024);   // about four non-leaf cells a thread on the fullest level
+        const int want = std::max(1, cap / 256);
         const int grid = std::max(1, std::min(per_sm * c->sm_count, want));
         int lev_hi = g.levels - 1;
         unsigned *barrier = reinterpret_cast<unsigned *>(t.lvl_cnt + 2 * TREE_LV_SLOTS);
         void *args[] = {&lev_hi, &t.lvl_cnt, &t.lvl_list, &barrier, &t.cell_off, &t.counters, &t.cap_cells,
                         &t.cells, &t.lvl8, &t.psum, &views};
-        OV_CUDA(c, cudaLaunchCooperativeKernel((const void *)k_levels, grid, 256, args, 0, s));
+        OV_CUDA(c, cudaLaunchCooperativeKernel((const void *)k_levels, grid, kLevelThreads, args, 0, s));
     }
-    k_root<<<nt, 256, 0, s>>>(t.order, t.cell_off, t.counters, t.tt, t.nm, g, t.cells, t.psum, t.first, t.cap_cells,
+    k_root<<<nt, 256, 0, s>>>(t.order, t.cell_off, t.counters, t.tt, t.nm, g, t.cells, t.lvl8, t.psum, t.first, t.cap_cells,
                               views);
     c->launches += 3;
     OV_CUDA(c, cudaGetLastError());
