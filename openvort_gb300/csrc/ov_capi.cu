@@ -163,7 +163,7 @@ static void release_buffers(ov_ctx *c)
     ov_tree_free(c->tree);
     void *dev[] = {c->fwd, c->rev, c->status, c->pin, c->dnodes, c->d_tid, c->d_qorder, c->d_tprm, c->d_mrange,
                    c->d_pairs, c->d_npairs, c->d_loop_off, c->d_loop_nodes, c->d_loop_buf, c->d_loop_cut,
-                   c->rec_nodes, c->rec_pair, c->rec_out, c->rec_corr, c->rec_part, c->rec_split, c->rec_seg, c->rec_far, c->near_lists, c->fft_buf,
+                   c->rec_nodes, c->rec_pair, c->rec_out, c->rec_corr, c->rec_part, c->rec_split, c->rec_seg, c->rec_far, c->near_lists, c->lia, c->fft_buf,
                    c->fft_tw, c->long_buf, c->d_rm, c->d_rm_lim, c->dsum, c->part, c->d_node_counts, c->flush_buf,
                    c->d_stage, c->d_time};
     for (void *p : dev)
@@ -184,6 +184,8 @@ static void release_buffers(ov_ctx *c)
     c->rec_far = nullptr;
     c->near_lists = nullptr;
     c->near_warps = 0;
+    c->lia = nullptr;
+    c->lia_cap = 0;
     c->fft_buf = c->fft_tw = nullptr;
     c->long_buf = nullptr;
     c->d_rm = nullptr;
@@ -976,20 +978,21 @@ static int eval_async(ov_ctx *c, NodeArrays &na, double t, bool tangents, cudaSt
     const bool ph = c->phase_timing && (c->time_dev_index < 0 || in_graph);
     const unsigned ev_flags = in_graph ? cudaEventRecordExternal : cudaEventRecordDefault;
     if (ph) OV_CUDA(c, cudaEventRecordWithFlags(c->ph[0], s, ev_flags));
+    int r = ov_reserve_velocity_scratch(c);
+    if (r) return r;
     if (tangents) {
         OV_CUDA(c, cudaEventRecord(c->fork_ev, s));
         OV_CUDA(c, cudaStreamWaitEvent(c->side, c->fork_ev, 0));
-        ov_launch_tangents(c, na, c->side);
+        ov_launch_tangents(c, na, true, c->side);
         if (ph) OV_CUDA(c, cudaEventRecordWithFlags(c->ph[1], c->side, ev_flags));
         OV_CUDA(c, cudaEventRecord(c->join_ev, c->side));
     } else if (ph) {
         OV_CUDA(c, cudaEventRecordWithFlags(c->ph[1], s, ev_flags));
     }
-    int r = ov_tree_build(c, na, s);
-    if (r) return r;
+    if ((r = ov_tree_build(c, na, s))) return r;
     if (ph) OV_CUDA(c, cudaEventRecordWithFlags(c->ph[2], s, ev_flags));
     if (tangents) OV_CUDA(c, cudaStreamWaitEvent(s, c->join_ev, 0));
-    if ((r = ov_launch_velocities(c, na, t, c->precision, s))) return r;
+    if ((r = ov_launch_velocities(c, na, t, c->precision, tangents, s))) return r;
     if (ph) OV_CUDA(c, cudaEventRecordWithFlags(c->ph[3], s, ev_flags));
     OV_CUDA(c, cudaGetLastError());
     return OV_OK;
@@ -1067,7 +1070,7 @@ int ov_update_tangents_normals(ov_ctx *c)
     int r = check_ready(c);
     if (r) return r;
     OV_CUDA(c, cudaMemsetAsync(c->tree.counters, 0, TC_WORDS * 4, c->stream));
-    ov_launch_tangents(c, c->node, c->stream);   // (all counter words cleared: a new call)
+    ov_launch_tangents(c, c->node, false, c->stream);   // (all counter words cleared: a new call)
     OV_CUDA(c, cudaGetLastError());
     if ((r = collect_stats(c, true))) return r;
     return error_from_word(c);
@@ -1131,8 +1134,8 @@ static unsigned long long graph_key(ov_ctx *c)
         h = mix64(h, lay, sizeof lay);
         h = mix64(h, &m.params, sizeof m.params);
     }
-    const void *ptrs[10] = {c->node.x, c->tree.cells, c->part, c->d_time, c->d_tid, c->d_tprm, c->d_qorder, c->d_mrange,
-                           c->tree.tt, c->near_lists};
+    const void *ptrs[11] = {c->node.x, c->tree.cells, c->part, c->d_time, c->d_tid, c->d_tprm, c->d_qorder, c->d_mrange,
+                           c->tree.tt, c->near_lists, c->lia};
     h = mix64(h, ptrs, sizeof ptrs);
     return h;
 }

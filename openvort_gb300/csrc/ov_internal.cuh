@@ -276,6 +276,8 @@ struct ov_ctx {
     CellFX *rec_seg = nullptr;       // fixed-point segments of the FP64 direct sums
     int *near_lists = nullptr;       // the mixed traversals' deferred cells
     size_t near_warps = 0;
+    double *lia = nullptr;           // local velocities of an evaluation (3 arrays of lia_cap)
+    int lia_cap = 0;
     float4 *rec_far = nullptr;       // segments of the candidates' far sums
     int rec_seg_cap = 0, rec_far_cap = 0;
     double *h_corr = nullptr;    // pinned host copy of the corrections
@@ -374,8 +376,8 @@ void ov_scan_exclusive(ov_ctx *c, const int *in, int *out, int n_max, const int 
                        int *tmp, cudaStream_t s);
 
 // velocity path (ov_velocity.cu)
-void ov_launch_tangents(ov_ctx *c, const NodeArrays &na, cudaStream_t s);
-int ov_launch_velocities(ov_ctx *c, const NodeArrays &na, double t, int precision, cudaStream_t s);
+void ov_launch_tangents(ov_ctx *c, const NodeArrays &na, bool lia, cudaStream_t s);
+int ov_launch_velocities(ov_ctx *c, const NodeArrays &na, double t, int precision, bool lia, cudaStream_t s);
 int ov_reserve_velocity_scratch(ov_ctx *c);
 int ov_query_groups(ov_ctx *c);
 int ov_traversal_blocks(ov_ctx *c, int precision, int warps, int *per_sm);

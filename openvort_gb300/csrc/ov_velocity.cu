@@ -38,6 +38,8 @@ struct VelArgs {
     const DevParams *tprm;  // per-member parameters (null: prm)
     const int2 *mrange;     // per-member slot range [x, y) (null: [0, cap))
     int *work;              // work-queue counter
+    double *lia;            // local velocities of k_tangents, 3 arrays of cap (null: not computed)
+    int one_sum;            // the traversal writes one sum per group (mixed), not own point and images
     int *near_lists;        // mixed traversals: kNearCap * 32 deferred cells a warp of the grid
     int nt;                 // members
     int G;                  // query groups per node
@@ -197,10 +199,33 @@ __device__ __forceinline__ double wrapped_len(const Geometry &g, const double r1
     return len3_ref(rn_sub(r1[0], r2[0]), rn_sub(r1[1], r2[1]), rn_sub(r1[2], r2[2]));
 }
 
+// Local velocity t x n f (LIA, tangle.c:568-592) of a node between segments
+// of these lengths.
+__device__ __forceinline__ void local_vel(const DevParams &P, double l_next, double l_prev, const double tg[3],
+                                          const double nm[3], double vs[3])
+{
+    double f = rn_div(rn_div(rn_mul(P.kappa,
+                              log(rn_div(rn_div(rn_mul(2.0, sqrt(rn_mul(l_next, l_prev))), sqrt(M_E)), P.a0))),
+                         4.0),
+                    M_PI);
+    vs[0] = rn_mul(rn_sub(rn_mul(tg[1], nm[2]), rn_mul(tg[2], nm[1])), f);
+    vs[1] = rn_mul(rn_sub(rn_mul(tg[2], nm[0]), rn_mul(tg[0], nm[2])), f);
+    vs[2] = rn_mul(rn_sub(rn_mul(tg[0], nm[1]), rn_mul(tg[1], nm[0])), f);
+}
+
+// Mark of a node whose local velocity k_tangents could not compute (a NaN that
+// no operation gives): k_vel_finish computes it, or reports the broken walk.
+constexpr long long kNoLia = 0x7ff9c0de00000001ll;
+
+// With a.lia also the local velocities, which k_vel_finish adds: the logarithm,
+// the square roots and the divisions run here beside the tree build, not in the
+// chain after the traversal (k_vel_finish 29 to 15 us at 496 nodes, 37 to 14 at 65,536,
+// mixed; k_tangents 30 to 38 and 53 to 69, less than the build takes).
 __global__ void k_tangents(VelArgs a, int cap, int *counters)
 {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= cap || a.status[k] == OV_EMPTY) return;
+    if (a.lia) a.lia[k] = __longlong_as_double(kNoLia);
     const Geometry &g = a.geo;
     double s0[3] = {a.x[k], a.y[k], a.z[k]}, s1[3], s2[3], sm1[3], sm2[3];
     bool ok = step_node_dev(a, k, 1, s1) & step_node_dev(a, k, 2, s2) & step_node_dev(a, k, -1, sm1) &
@@ -263,6 +288,16 @@ __global__ void k_tangents(VelArgs a, int cap, int *counters)
     double *Nn[3] = {(double *)a.nx, (double *)a.ny, (double *)a.nz};
 #pragma unroll
     for (int ax = 0; ax < 3; ++ax) { T[ax][k] = tg[ax]; Nn[ax][k] = nm[ax]; }
+    if (a.lia) {
+        const int m = a.tprm ? a.tid[k] : 0;
+        if (a.tprm && (m < 0 || m >= a.nt)) return;
+        // (d1 is the length to the next node; the previous segment's is taken
+        // from the previous node, as everywhere)
+        double vs[3];
+        local_vel(a.tprm ? a.tprm[m] : a.prm, d1, wrapped_len(g, sm1, s0), tg, nm, vs);
+#pragma unroll
+        for (int ax = 0; ax < 3; ++ax) a.lia[(size_t)ax * a.cap + k] = vs[ax];
+    }
 }
 
 __device__ __forceinline__ double now(const VelArgs &a) { return a.t_dev ? a.t_dev[a.t_index] : a.t; }
@@ -288,7 +323,6 @@ __device__ __forceinline__ void image_point(const Geometry &g, int j, const doub
     for (int m = 0; m < g.nreflect[j]; ++m) {
         const int f = g.reflect[j][m];
         if (f < 0 || f > 5) continue;
-        // (selected, not indexed: the arrays stay in registers)
         int ax = f >> 1;
         double w = (f & 1) ? g.hi[ax] : g.lo[ax];
         q[ax] = rn_sub(rn_mul(2.0, w), p[ax]);
@@ -419,21 +453,23 @@ __device__ __forceinline__ bool finish_impl(const VelArgs &a, const DevParams &P
         vs_out[0] = vs_out[1] = vs_out[2] = 0;
         return true;
     }
-    double nx_[3], pv[3];
-    if (!(step_node_dev(a, id, 1, nx_) && step_node_dev(a, id, -1, pv))) {
-        *err |= OV_EW_WALK;
-        return false;
+    double vs[3], tg[3] = {0, 0, 0};
+    if (P.friction || !a.lia) { tg[0] = a.tx[id]; tg[1] = a.ty[id]; tg[2] = a.tz[id]; }
+    bool have = false;
+    if (a.lia) {
+        for (int ax = 0; ax < 3; ++ax) vs[ax] = a.lia[(size_t)ax * a.cap + id];
+        have = __double_as_longlong(vs[0]) != kNoLia;
     }
-    double l_next = wrapped_len(a.geo, p, nx_);
-    double l_prev = wrapped_len(a.geo, pv, p);
-    double f = rn_div(rn_div(rn_mul(P.kappa,
-                              log(rn_div(rn_div(rn_mul(2.0, sqrt(rn_mul(l_next, l_prev))), sqrt(M_E)), P.a0))),
-                         4.0),
-                    M_PI);
-    double tg[3] = {a.tx[id], a.ty[id], a.tz[id]}, nm[3] = {a.nx[id], a.ny[id], a.nz[id]};
-    double vs[3] = {rn_mul(rn_sub(rn_mul(tg[1], nm[2]), rn_mul(tg[2], nm[1])), f),
-                    rn_mul(rn_sub(rn_mul(tg[2], nm[0]), rn_mul(tg[0], nm[2])), f),
-                    rn_mul(rn_sub(rn_mul(tg[0], nm[1]), rn_mul(tg[1], nm[0])), f)};
+    if (!have) {
+        double nx_[3], pv[3];
+        if (!(step_node_dev(a, id, 1, nx_) && step_node_dev(a, id, -1, pv))) {
+            *err |= OV_EW_WALK;
+            return false;
+        }
+        tg[0] = a.tx[id]; tg[1] = a.ty[id]; tg[2] = a.tz[id];
+        const double nm[3] = {a.nx[id], a.ny[id], a.nz[id]};
+        local_vel(P, wrapped_len(a.geo, p, nx_), wrapped_len(a.geo, pv, p), tg, nm, vs);
+    }
     double ev[3];
     ext_vel(P.vs_type, P.vs_dir, P.vs_s1, P.vs_s0, P.vs_tld, now(a), ev);
     for (int ax = 0; ax < 3; ++ax) vs[ax] = rn_add(rn_add(rn_add(vs[ax], ev[ax]), prim[ax]), img[ax]);
@@ -573,7 +609,7 @@ __global__ void __launch_bounds__(32 * W, min_blocks<W>()) k_vel_fp64(VelArgs a,
         if (valid) {
             const size_t cap = (size_t)a.cap;
             for (int ax = 0; ax < 3; ++ax) {
-                part_out[((size_t)(2 * w.grp) * 3 + ax) * cap + tix] = prim[ax];
+                if (w.grp == 0) part_out[(size_t)ax * cap + tix] = prim[ax];
                 part_out[((size_t)(2 * w.grp + 1) * 3 + ax) * cap + tix] = img[ax];
             }
         }
@@ -595,18 +631,18 @@ __global__ void __launch_bounds__(32 * W, min_blocks<W>()) k_vel_fp64(VelArgs a,
 }
 
 // Parts of split walks: each group's S parts added in part order into its
-// first part's slot (one thread per group, component and target).
+// first part's slot (one thread per sum, component and target; the sums are the
+// node's own, of group 0, and the images' of each group).
 __global__ void k_part_sum(VelArgs a, double *__restrict__ part)
 {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const int nne = min(a.counters[TC_NNE], a.cap);
-    const long long per = 6LL * nne;
-    if (i >= per * a.G) return;
-    const int g = (int)(i / per);
-    const int r = (int)(i - (long long)g * per);
-    const int comp = r / nne, tix = r - comp * nne;   // comp: prim x,y,z then img x,y,z
+    const long long per = 3LL * nne;
+    if (i >= per * (a.G + 1)) return;
+    const int u = (int)(i / per), g = u == 0 ? 0 : u - 1, half = u > 0;
+    const int r = (int)(i - (long long)u * per);
+    const int ax = r / nne, tix = r - ax * nne;
     const size_t cap = (size_t)a.cap;
-    const int half = comp / 3, ax = comp - 3 * half;
     double s = 0;
     for (int k = 0; k < a.S; ++k) {
         const size_t gs = (size_t)g * a.S + k;
@@ -628,11 +664,17 @@ __global__ void k_vel_finish(VelArgs a, const double *__restrict__ part_in)
     const size_t cap = (size_t)a.cap;
     double prim[3] = {0, 0, 0}, img[3] = {0, 0, 0};
     // (with parts, k_part_sum has added each group's parts into its first)
-    for (int g = 0; g < a.G * a.S; g += a.S)
-        for (int ax = 0; ax < 3; ++ax) {
-            prim[ax] = rn_add(prim[ax], part_in[((size_t)(2 * g) * 3 + ax) * cap + tix]);
-            img[ax] = rn_add(img[ax], part_in[((size_t)(2 * g + 1) * 3 + ax) * cap + tix]);
-        }
+    // the first group alone has the node itself among its query points
+    for (int ax = 0; ax < 3; ++ax) prim[ax] = part_in[(size_t)ax * cap + tix];
+    if (a.one_sum) {
+        for (int g = 1; g < a.G; ++g)
+            for (int ax = 0; ax < 3; ++ax) prim[ax] = rn_add(prim[ax], part_in[((size_t)(2 * g) * 3 + ax) * cap + tix]);
+    } else {
+#pragma unroll 9
+        for (int g = 0; g < a.G; ++g)
+            for (int ax = 0; ax < 3; ++ax)
+                img[ax] = rn_add(img[ax], part_in[((size_t)(2 * g * a.S + 1) * 3 + ax) * cap + tix]);
+    }
     double p[3] = {a.x[id], a.y[id], a.z[id]};
     double vs[3], vel[3];
     int err = 0;
@@ -1133,7 +1175,6 @@ __global__ void __launch_bounds__(32 * W, (min_blocks_mixed<W, HI>())) k_vel_mix
             const size_t cap = (size_t)a.cap;
             for (int ax = 0; ax < 3; ++ax) {
                 part_out[((size_t)(2 * w.grp) * 3 + ax) * cap + tix] = bh[ax];
-                part_out[((size_t)(2 * w.grp + 1) * 3 + ax) * cap + tix] = 0.0;
             }
         }
         count_node(a, valid, id, m.nvis, m.nacc);
@@ -1369,7 +1410,6 @@ __global__ void __launch_bounds__(32 * W, (min_blocks_mixp<W, R>())) k_vel_mixp(
                                   acc_value(m.s2, m.c2) + w64[2]};
             for (int ax = 0; ax < 3; ++ax) {
                 part_out[((size_t)(2 * w.grp) * 3 + ax) * cap + tix] = bh[ax];
-                part_out[((size_t)(2 * w.grp + 1) * 3 + ax) * cap + tix] = 0.0;
             }
         }
         count_node(a, valid, id, m.nvis, m.nacc);
@@ -1710,7 +1750,7 @@ __global__ void __launch_bounds__(32 * W, min_blocks_split<W>()) k_vel_split(Vel
         }
         if (valid)
             for (int ax = 0; ax < 3; ++ax) {
-                if (!own) out[(size_t)ax * a.cap] = 0.0;
+                if (!own && w.grp == 0) out[(size_t)ax * a.cap] = 0.0;
                 out[(size_t)(3 + ax) * a.cap] = img[ax];
             }
         count_node(a, valid, id, m.nvis, m.nacc);
@@ -1761,6 +1801,9 @@ namespace {
 VelArgs make_args(ov_ctx *c, const NodeArrays &na, double t, unsigned long long *stat)
 {
     VelArgs a;
+    a.lia = nullptr;
+    a.one_sum = 0;
+    a.near_lists = nullptr;
     a.order = c->tree.torder;
     a.counters = c->tree.counters;
     a.cells = c->tree.cells;
@@ -1822,9 +1865,11 @@ VelArgs make_args(ov_ctx *c, const NodeArrays &na, double t, unsigned long long 
 
 }  // namespace
 
-void ov_launch_tangents(ov_ctx *c, const NodeArrays &na, cudaStream_t s)
+// (lia: also the local velocities, into c->lia)
+void ov_launch_tangents(ov_ctx *c, const NodeArrays &na, bool lia, cudaStream_t s)
 {
     VelArgs a = make_args(c, na, 0.0, nullptr);
+    if (lia) a.lia = c->lia;
     k_tangents<<<(c->cap + 255) / 256, 256, 0, s>>>(a, c->cap, c->tree.counters);
     c->launches++;
 }
@@ -1891,6 +1936,13 @@ int ov_reserve_velocity_scratch(ov_ctx *c)
         c->part = nullptr;
         OV_ALLOC(c, cudaMalloc(&c->part, need * sizeof(double)));
         c->part_cap = need;
+    }
+    if (c->lia_cap < c->cap) {
+        if (c->lia) cudaFree(c->lia);
+        c->lia = nullptr;
+        c->lia_cap = 0;
+        OV_ALLOC(c, cudaMalloc(&c->lia, 3 * (size_t)c->cap * sizeof(double)));
+        c->lia_cap = c->cap;
     }
     if (c->precision == OV_PREC_MIXED) {
         const int warps = launch_warps(c), r = reserve_near_lists(c, (size_t)ov_traversal_blocks(c, c->precision, warps, nullptr) * warps);
@@ -1961,10 +2013,13 @@ int ov_traversal_blocks(ov_ctx *c, int precision, int warps, int *per_sm)
     return (int)std::max(1LL, blocks);
 }
 
-int ov_launch_velocities(ov_ctx *c, const NodeArrays &na, double t, int precision, cudaStream_t s)
+// (lia: c->lia has the local velocities of these nodes, from ov_launch_tangents)
+int ov_launch_velocities(ov_ctx *c, const NodeArrays &na, double t, int precision, bool lia, cudaStream_t s)
 {
     VelArgs a = make_args(c, na, t, ov_stat_ptr(c));
     a.S = ov_sub_walks(c, precision);
+    a.lia = lia ? c->lia : nullptr;
+    a.one_sum = precision == OV_PREC_MIXED;
     if (c->time_dev_index >= 0) {
         a.t_dev = c->d_time;
         a.t_index = c->time_dev_index;
@@ -1986,7 +2041,6 @@ int ov_launch_velocities(ov_ctx *c, const NodeArrays &na, double t, int precisio
         OV_CUDA(c, cudaMemsetAsync(c->d_node_counts, 0, need * sizeof(unsigned), s));
         a.node_counts = c->d_node_counts;
     }
-    a.near_lists = nullptr;
     if (precision == OV_PREC_MIXED) {
         if ((r = reserve_near_lists(c, (size_t)blocks * warps))) return r;
         a.near_lists = c->near_lists;
@@ -1995,7 +2049,7 @@ int ov_launch_velocities(ov_ctx *c, const NodeArrays &na, double t, int precisio
     vel_kernel(precision, ov_split_walk(c, precision), warps, mixed_variant(c), has_mirror_images(c->geo))<<<
         blocks, 32 * warps, list_bytes(c, precision, warps), s>>>(a, c->part);
     if (a.S > 1) {
-        const long long threads = 6LL * c->cap * a.G;
+        const long long threads = 3LL * c->cap * (a.G + 1);
         k_part_sum<<<(unsigned)((threads + 127) / 128), 128, 0, s>>>(a, c->part);
         c->launches++;
     }
