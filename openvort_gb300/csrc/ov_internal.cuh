@@ -372,6 +372,7 @@ inline int ov_fx_bits(const ov_ctx *c) { return c->geo.sph ? 38 : 39; }
 
 // sort / scan (ov_sort.cu)
 void ov_sort_keys(ov_ctx *c, TreeBuf &t, int n, cudaStream_t s);
+bool ov_sort_by_rank(int n);
 void ov_scan_exclusive(ov_ctx *c, const int *in, int *out, int n_max, const int *n_dev, int add,
                        int *tmp, cudaStream_t s);
 

@@ -1289,8 +1289,8 @@ int find_pairs(ov_ctx *c, std::vector<std::pair<int, int>> &out)
     if (r) return r;
     TreeBuf &t = c->tree;
     int nb = (cap + 255) / 256;
-    k_grid_keys<<<nb, 256, 0, c->stream>>>(c->status, c->node.x, c->node.y, c->node.z, c->n_live, cap, gg, t.keys,
-                                           t.order);
+    k_grid_keys<<<nb, 256, 0, c->stream>>>(c->status, c->node.x, c->node.y, c->node.z, c->n_live, cap, gg,
+                                           ov_sort_by_rank(cap) ? t.keys_alt : t.keys, t.order);
     c->launches++;
     ov_sort_keys(c, t, cap, c->stream);
     for (int attempt = 0; attempt < 2; ++attempt) {

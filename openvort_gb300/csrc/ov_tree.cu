@@ -1049,11 +1049,12 @@ int ov_tree_build(ov_ctx *c, const NodeArrays &na, cudaStream_t s)
     OV_CUDA(c, cudaMemsetAsync(t.tt, 0, (size_t)nt * TT_WORDS * 4, s));
     OV_CUDA(c, cudaMemsetAsync(t.lvl_cnt, 0, 3 * TREE_LV_SLOTS * 4, s));
     int nb = (cap + 255) / 256;
+    uint64_t *unsorted = ov_sort_by_rank(cap) ? t.keys_alt : t.keys;
     if (c->geo.sph)
-        k_keys<true><<<nb, 256, 0, s>>>(c->status, na.x, na.y, na.z, nt > 1 ? c->d_tid : nullptr, cap, g, t.keys,
+        k_keys<true><<<nb, 256, 0, s>>>(c->status, na.x, na.y, na.z, nt > 1 ? c->d_tid : nullptr, cap, g, unsorted,
                                         t.order, t.counters, t.tt, c->fwd, c->geo, t.nm);
     else
-        k_keys<false><<<nb, 256, 0, s>>>(c->status, na.x, na.y, na.z, nt > 1 ? c->d_tid : nullptr, cap, g, t.keys,
+        k_keys<false><<<nb, 256, 0, s>>>(c->status, na.x, na.y, na.z, nt > 1 ? c->d_tid : nullptr, cap, g, unsorted,
                                          t.order, t.counters, t.tt, c->fwd, c->geo, t.nm);
     k_layout<<<1, 32, 0, s>>>(t.tt, nt, c->d_qorder, t.counters, t.lev_tab, g.root_lm, c->params.bh_resolution);
     c->launches += 2;

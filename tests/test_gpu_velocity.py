@@ -252,3 +252,30 @@ def test_decreasing_flow_vs_oracle(port, time):
     port.rk4_step(t, time, 5e-5)
     assert rel_err(pos, t.copy("pos")) < FP64_TOL
     t.free()
+
+
+@pytest.mark.parametrize("n", [2, 33, 2048, 2049, 8192])
+def test_rank_sorted_tree_is_the_radix_sorted_tree(n):
+    """Up to 8,192 slots the keys are sorted by rank: the same tree (cells, decisions)
+    and the same velocities, up to the order of the partial sums, as behind enough
+    EMPTY slots for the radix passes; with coincident nodes, which tie."""
+    base = W.random_walk_tangle(1, n, D=0.1, seed=9)
+    pos = np.array(base.pos)
+    pos[n // 2::7] = pos[n // 3]
+    got = []
+    for pad in (0, 9000):
+        fwd, rev = np.full(n + pad, -1, np.int32), np.full(n + pad, -1, np.int32)
+        fwd[:n], rev[:n] = base.conn[:, 0], base.conn[:, 1]
+        status = np.full(n + pad, abi.OV_EMPTY, np.int32)
+        status[:n] = abi.OV_FREE
+        ht = W.HostTangle(np.concatenate([pos, np.zeros((pad, 3))]), fwd, rev, base.box_lo, base.box_hi, status=status)
+        ctx = gpu.Context(0, params=W.config_params("rw"), precision=abi.OV_PREC_MIXED)
+        ctx.set_tuning(query_groups=4)
+        ctx.upload(ht)
+        ctx.update_tangle(0.0)
+        ctx.download(ht)
+        st = ctx.stats()
+        ctx.close()
+        got.append((np.array(ht.vs[:n]), [st[k] for k in ("cells", "max_depth", "visits", "accepts", "error_word")]))
+    assert got[0][1] == got[1][1]
+    np.testing.assert_array_equal(got[0][0], got[1][0])
