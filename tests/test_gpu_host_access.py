@@ -62,3 +62,24 @@ def test_download_into_a_larger_host_tangle():
         assert np.all(big.vels[ht.n:] == 0) and np.all(big.stat[ht.n:, 0] == abi.OV_EMPTY)
     for a, b in zip(*outs):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("n", [3, 255, 256, 257, 769])
+@pytest.mark.parametrize("direct", [False, True])
+def test_round_trip_at_block_edges(n, direct):
+    """What is uploaded is what is downloaded, for the last slots of a block too;
+    the slots behind the tangle's are left alone."""
+    ht = W.random_walk_tangle(1, n, D=0.1, seed=6)
+    rng = np.random.default_rng(n)
+    for k in FIELDS[1:5]:
+        getattr(ht, k)[:] = rng.standard_normal((n, 3))
+    want = {k: np.array(getattr(ht, k)) for k in FIELDS}
+    ctx = gpu.Context(0, params=W.config_params("rw"))
+    ctx.set_host_access(direct)
+    ctx.upload(ht)
+    for k in FIELDS[:5]:
+        getattr(ht, k)[:] = 0
+    ctx.download(ht)
+    ctx.close()
+    for k in FIELDS:
+        np.testing.assert_array_equal(getattr(ht, k), want[k], err_msg=k)
