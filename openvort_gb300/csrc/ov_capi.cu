@@ -484,10 +484,11 @@ static HostView stage_view(char *stage, int n)
 // sectors (the four result fields of 65,536 nodes: 39 us, 124 that way).
 constexpr int kPackThreads = 256;
 
-// Host layout (vec3 fields, ov_neighbour, ov_node_status) -> device arrays for
-// slots [0, cap): slots past n get zeros, -1 links, EMPTY, no wall.
-__global__ void __launch_bounds__(kPackThreads) k_unpack(HostView src, unsigned fields, unsigned have, int n, int cap,
-                                                         NodePtrs d)
+// Host layout (vec3 fields, ov_neighbour, ov_node_status) of n slots -> device
+// slots [lo, lo + cap), links shifted by lo: slots past n get zeros, -1 links,
+// EMPTY, no wall.
+__global__ void __launch_bounds__(kPackThreads) k_unpack(HostView src, unsigned fields, unsigned have, int n, int lo,
+                                                         int cap, NodePtrs d)
 {
     __shared__ double buf[3 * kPackThreads];
     const int k0 = blockIdx.x * kPackThreads, k = k0 + threadIdx.x;
@@ -505,15 +506,16 @@ __global__ void __launch_bounds__(kPackThreads) k_unpack(HostView src, unsigned 
         }
         __syncthreads();
         if (k < cap)
-            for (int a = 0; a < 3; ++a) d.d[3 * f + a][k] = buf[3 * threadIdx.x + a];
+            for (int a = 0; a < 3; ++a) d.d[3 * f + a][lo + k] = buf[3 * threadIdx.x + a];
         __syncthreads();
     }
     if ((fields & OV_F_TOPOLOGY) && k < cap) {
         const bool in = k < n;
-        d.fwd[k] = in ? src.con[k].forward : -1;
-        d.rev[k] = in ? src.con[k].reverse : -1;
-        d.status[k] = in ? src.st[k].status : OV_EMPTY;
-        d.pin[k] = in ? src.st[k].pin_wall : OV_NOT_A_FACE;
+        const int f = in ? src.con[k].forward : -1, b = in ? src.con[k].reverse : -1;
+        d.fwd[lo + k] = f >= 0 ? f + lo : -1;
+        d.rev[lo + k] = b >= 0 ? b + lo : -1;
+        d.status[lo + k] = in ? src.st[k].status : OV_EMPTY;
+        d.pin[lo + k] = in ? src.st[k].pin_wall : OV_NOT_A_FACE;
     }
 }
 
@@ -676,6 +678,45 @@ int ov_move_device_slots(ov_ctx *c, const std::vector<Member> &old)
     return OV_OK;
 }
 
+// A host tangle's arrays into device slots [lo, lo + span).  The transposition
+// (k_unpack) reads the caller's arrays in place when the device reads pageable
+// host memory, else one copy of each into the device stage.
+static int unpack_tangle(ov_ctx *c, const ov_tangle_state *t, unsigned fields, int lo, int span)
+{
+    const int n = t->N;
+    const ov_vec3 *src[5] = {t->vnodes, t->vels, t->vs, t->tangents, t->normals};
+    const unsigned bits[5] = {OV_F_POS, OV_F_VELS, OV_F_VS, OV_F_TANGENTS, OV_F_NORMALS};
+    const bool direct = c->pageable && c->host_direct;
+    HostView view = {};
+    if (direct) {
+        for (int f = 0; f < 5; ++f) view.f[f] = const_cast<ov_vec3 *>(src[f]);
+        view.con = t->connections;
+        view.st = t->status;
+    } else {
+        const size_t bytes = stage_topo_off(n) + (size_t)n * 16;
+        int r = ensure_dstage(c, std::max(bytes, (size_t)16));
+        if (r) return r;
+        view = stage_view(c->d_stage, n);
+    }
+    unsigned have = 0;
+    for (int f = 0; f < 5; ++f)
+        if ((fields & bits[f]) && src[f] && n > 0) {
+            if (!direct)
+                OV_CUDA(c, cudaMemcpyAsync(view.f[f], src[f], (size_t)n * 24, cudaMemcpyHostToDevice, c->stream));
+            have |= bits[f];
+        }
+    if ((fields & OV_F_TOPOLOGY) && n > 0 && !direct) {
+        OV_CUDA(c, cudaMemcpyAsync(view.con, t->connections, (size_t)n * 8, cudaMemcpyHostToDevice, c->stream));
+        OV_CUDA(c, cudaMemcpyAsync(view.st, t->status, (size_t)n * 8, cudaMemcpyHostToDevice, c->stream));
+    }
+    if (span <= 0) return OV_OK;
+    k_unpack<<<(span + kPackThreads - 1) / kPackThreads, kPackThreads, 0, c->stream>>>(view, fields, have, n, lo, span,
+                                                                                      node_ptrs(c));
+    c->launches++;
+    OV_CUDA(c, cudaGetLastError());
+    return OV_OK;
+}
+
 extern "C" {
 
 int ov_upload_ensemble(ov_ctx *c, const ov_tangle_state *const *ts, const ov_params *params, int n,
@@ -729,39 +770,8 @@ int ov_upload_ensemble(ov_ctx *c, const ov_tangle_state *const *ts, const ov_par
     set_geometry(c, ts[0]->box, ts[0]->bimg);
     if ((r = ov_upload_member_tables(c))) return r;
     size_t cap = (size_t)c->cap;
-    if ((r = ensure_stage(c, cap * 3 * sizeof(double) * 5 + cap * 4 * sizeof(int)))) return r;
-    double *h = c->h_stage;
-    int *hi = (int *)(h + 15 * cap);
-    std::fill(h, h + 15 * cap, 0.0);
-    std::fill(hi, hi + 2 * cap, -1);
-    std::fill(hi + 2 * cap, hi + 3 * cap, (int)OV_EMPTY);
-    std::fill(hi + 3 * cap, hi + 4 * cap, (int)OV_NOT_A_FACE);
-    for (int i = 0; i < n; ++i) {
-        const ov_tangle_state *t = ts[i];
-        const size_t o = (size_t)mem[i].lo;
-        const ov_vec3 *src[5] = {t->vnodes, t->vels, t->vs, t->tangents, t->normals};
-        for (int f = 0; f < 5; ++f) {
-            if (!src[f]) continue;
-            double *dst = h + 3 * cap * f;
-            for (int a = 0; a < 3; ++a)
-                for (int k = 0; k < t->N; ++k) dst[a * cap + o + k] = src[f][k].p[a];
-        }
-        for (int k = 0; k < t->N; ++k) {
-            int f = t->connections[k].forward, b = t->connections[k].reverse;
-            hi[o + k] = f >= 0 ? f + (int)o : -1;
-            hi[cap + o + k] = b >= 0 ? b + (int)o : -1;
-            hi[2 * cap + o + k] = t->status[k].status;
-            hi[3 * cap + o + k] = t->status[k].pin_wall;
-        }
-    }
-    double *dd[15] = {c->node.x, c->node.y, c->node.z, c->node.vx, c->node.vy, c->node.vz,
-                      c->node.sx, c->node.sy, c->node.sz, c->node.tx, c->node.ty, c->node.tz,
-                      c->node.nx, c->node.ny, c->node.nz};
-    for (int k = 0; k < 15; ++k)
-        OV_CUDA(c, cudaMemcpyAsync(dd[k], h + k * cap, cap * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    int *di[4] = {c->fwd, c->rev, c->status, c->pin};
-    for (int i = 0; i < 4; ++i)
-        OV_CUDA(c, cudaMemcpyAsync(di[i], hi + i * cap, cap * sizeof(int), cudaMemcpyHostToDevice, c->stream));
+    for (int i = 0; i < n; ++i)   // the last member's launch also empties the slots behind the pool
+        if ((r = unpack_tangle(c, ts[i], OV_F_ALL, mem[i].lo, i + 1 < n ? mem[i].cap : (int)cap - mem[i].lo))) return r;
     c->last_h2d = cap * (15 * sizeof(double) + 4 * sizeof(int));
     OV_CUDA(c, cudaStreamSynchronize(c->stream));
     c->uploaded = true;
@@ -813,41 +823,11 @@ int ov_upload_tangle_fields(ov_ctx *c, const ov_tangle_state *t, unsigned fields
                 return ov_fail(c, OV_ERR_TOPOLOGY, "node %d: connections (%d,%d) / status %d out of range", k, f, b, st);
         }
     }
-    // the transposition to the device's arrays (k_unpack) reads the caller's
-    // arrays in place when the device reads pageable host memory, else one
-    // copy of each into the device stage
-    const ov_vec3 *src[5] = {t->vnodes, t->vels, t->vs, t->tangents, t->normals};
-    const unsigned bits[5] = {OV_F_POS, OV_F_VELS, OV_F_VS, OV_F_TANGENTS, OV_F_NORMALS};
-    const bool direct = c->pageable && c->host_direct;
-    HostView view = {};
-    if (direct) {
-        for (int f = 0; f < 5; ++f) view.f[f] = const_cast<ov_vec3 *>(src[f]);
-        view.con = t->connections;
-        view.st = t->status;
-    } else {
-        const size_t bytes = stage_topo_off(n) + (size_t)n * 16;
-        if ((r = ensure_dstage(c, std::max(bytes, (size_t)16)))) return r;
-        view = stage_view(c->d_stage, n);
-    }
-    unsigned have = 0;
+    if ((r = unpack_tangle(c, t, fields, 0, (int)cap))) return r;
     c->last_h2d = 0;
-    for (int f = 0; f < 5; ++f) {
-        if (!(fields & bits[f])) continue;
-        if (src[f] && n > 0) {
-            if (!direct)
-                OV_CUDA(c, cudaMemcpyAsync(view.f[f], src[f], (size_t)n * 24, cudaMemcpyHostToDevice, c->stream));
-            have |= bits[f];
-        }
-        c->last_h2d += 3 * cap * sizeof(double);
-    }
-    if ((fields & OV_F_TOPOLOGY) && n > 0 && !direct) {
-        OV_CUDA(c, cudaMemcpyAsync(view.con, t->connections, (size_t)n * 8, cudaMemcpyHostToDevice, c->stream));
-        OV_CUDA(c, cudaMemcpyAsync(view.st, t->status, (size_t)n * 8, cudaMemcpyHostToDevice, c->stream));
-    }
+    for (unsigned bit : {OV_F_POS, OV_F_VELS, OV_F_VS, OV_F_TANGENTS, OV_F_NORMALS})
+        if (fields & bit) c->last_h2d += 3 * cap * sizeof(double);
     if (fields & OV_F_TOPOLOGY) c->last_h2d += 4 * cap * sizeof(int);
-    k_unpack<<<(unsigned)((cap + kPackThreads - 1) / kPackThreads), kPackThreads, 0, c->stream>>>(view, fields, have, n, (int)cap, node_ptrs(c));
-    c->launches++;
-    OV_CUDA(c, cudaGetLastError());
     OV_CUDA(c, cudaStreamSynchronize(c->stream));
     c->uploaded = true;
     return OV_OK;

@@ -83,3 +83,28 @@ def test_round_trip_at_block_edges(n, direct):
     ctx.close()
     for k in FIELDS:
         np.testing.assert_array_equal(getattr(ht, k), want[k], err_msg=k)
+
+
+def test_ensemble_upload_in_place_equals_staged():
+    """Members of different sizes, with headroom: positions, links and status of each
+    member and the velocities of an evaluation, on both paths."""
+    outs = []
+    for direct in (False, True):
+        members = [W.random_walk_tangle(m, 50 + m, D=0.1, seed=m) for m in (1, 6, 3)]
+        ctx = gpu.Context(0, params=W.config_params("rw"))
+        ctx.set_host_access(direct)
+        ctx.upload_ensemble(members, [W.config_params("rw") for _ in members], 1.5)
+        ctx.update_tangle(0.0)
+        got = []
+        for i, m in enumerate(members):
+            want = np.array(m.pos), np.array(m.conn)
+            m.pos[:] = 0
+            h = ctx.download_member(i)
+            np.testing.assert_array_equal(h.pos[:len(want[0])], want[0])
+            np.testing.assert_array_equal(h.conn[:len(want[1])], want[1])
+            assert np.all(h.stat[len(want[0]):, 0] == abi.OV_EMPTY)
+            got.append(np.array(h.vels))
+        ctx.close()
+        outs.append(got)
+    for a, b in zip(*outs):
+        np.testing.assert_array_equal(a, b)
