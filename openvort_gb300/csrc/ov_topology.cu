@@ -358,6 +358,32 @@ __device__ __forceinline__ int lower_key(const uint64_t *keys, int n, uint64_t v
     return lo;
 }
 
+// True only when the two points are further apart than rec_dist by far more
+// than FP32 rounds: the difference wrapped in FP32 is within 2^-23 of 100 box
+// lengths, and the margin is 2e-5 of one.  (NaN: false.)
+__device__ __forceinline__ bool clearly_apart(const Geometry &geo, const double p[3], const double q[3],
+                                              double rec_dist)
+{
+    float d2 = 0, Lmax = 0;
+    bool sure = true;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const float L = (float)geo.L[a];
+        float d = (float)rn_sub(q[a], p[a]);
+        sure = sure && fabsf(d) < 100.0f * L;
+        if (geo.periodic[a]) d -= L * rintf(d / L);
+        d2 = fmaf(d, d, d2);
+        Lmax = fmaxf(Lmax, L);
+    }
+    const float far = (float)rec_dist * 1.00001f + 2e-5f * Lmax;
+    return sure && d2 > far * far;
+}
+
+// Candidate pairs, a thread per node.  Bound: chains of dependent loads.  Ten or so
+// searches of the sorted keys a thread (the 27 neighbouring cells each took two),
+// and few of the nodes found are close enough for the FP64 distance.
+// 122,000 nodes in 12 members: 490 us with two searches a cell, 200 with one a
+// row, 100 with the FP32 test before the distance.
 __global__ void k_pairs(const uint64_t *__restrict__ keys, const int *__restrict__ idx, int cap,
                         const double *__restrict__ x, const double *__restrict__ y, const double *__restrict__ z,
                         GridGeom gg, Geometry geo, double rec_dist, const int *__restrict__ tid,
@@ -374,31 +400,36 @@ __global__ void k_pairs(const uint64_t *__restrict__ keys, const int *__restrict
     int c[3] = {(int)(cid % gg.n[0]), (int)((cid / gg.n[0]) % gg.n[1]), (int)(cid / ((uint64_t)gg.n[0] * gg.n[1]))};
     double pk[3] = {x[k], y[k], z[k]};
     int lo3[3], hi3[3];
-    for (int a = 0; a < 3; ++a) {
+    for (int a = 1; a < 3; ++a) {
         if (gg.n[a] >= 3) { lo3[a] = -1; hi3[a] = 1; }
         else if (gg.n[a] == 2) { lo3[a] = 0; hi3[a] = 1; }
         else { lo3[a] = 0; hi3[a] = 0; }
     }
+    // the cells of a row (y, z) are neighbours in key order: one range, and a
+    // second one where the row wraps around
+    const int x0 = gg.n[0] >= 3 ? max(c[0] - 1, 0) : 0, x1 = gg.n[0] >= 3 ? min(c[0] + 1, gg.n[0] - 1) : gg.n[0] - 1;
+    const int xw = gg.n[0] >= 3 && gg.periodic[0] ? (c[0] == 0 ? gg.n[0] - 1 : c[0] == gg.n[0] - 1 ? 0 : -1) : -1;
     for (int dz = lo3[2]; dz <= hi3[2]; ++dz)
-        for (int dy = lo3[1]; dy <= hi3[1]; ++dy)
-            for (int dx = lo3[0]; dx <= hi3[0]; ++dx) {
-                int nc[3] = {c[0] + dx, c[1] + dy, c[2] + dz};
-                bool skip = false;
-                for (int a = 0; a < 3; ++a) {
-                    if (gg.n[a] <= 2) { nc[a] = ((nc[a] % gg.n[a]) + gg.n[a]) % gg.n[a]; continue; }
-                    if (nc[a] < 0 || nc[a] >= gg.n[a]) {
-                        if (!gg.periodic[a]) skip = true;
-                        nc[a] = (nc[a] + gg.n[a]) % gg.n[a];
-                    }
+        for (int dy = lo3[1]; dy <= hi3[1]; ++dy) {
+            int nc[3] = {0, c[1] + dy, c[2] + dz};
+            bool skip = false;
+            for (int a = 1; a < 3; ++a) {
+                if (gg.n[a] <= 2) { nc[a] = ((nc[a] % gg.n[a]) + gg.n[a]) % gg.n[a]; continue; }
+                if (nc[a] < 0 || nc[a] >= gg.n[a]) {
+                    if (!gg.periodic[a]) skip = true;
+                    nc[a] = (nc[a] + gg.n[a]) % gg.n[a];
                 }
-                if (skip) continue;
-                uint64_t ncid = ((uint64_t)nc[2] * gg.n[1] + nc[1]) * gg.n[0] + nc[0];
-                int b = lower_key(keys, cap, ncid << 32), e = lower_key(keys, cap, (ncid + 1) << 32);
-                for (int j = b; j < e; ++j) {
+            }
+            if (skip) continue;
+            const uint64_t row = ((uint64_t)nc[2] * gg.n[1] + nc[1]) * gg.n[0];
+            for (int part = 0; part < (xw >= 0 ? 2 : 1); ++part) {
+                const uint64_t first = (row + (part ? xw : x0)) << 32, last = (row + (part ? xw : x1) + 1) << 32;
+                for (int j = lower_key(keys, cap, first); j < cap && keys[j] < last; ++j) {
                     int l = idx[j];
                     if (l <= k) continue;
                     if (tid && tid[l] != mk) continue;
                     double v2[3] = {x[l], y[l], z[l]};
+                    if (clearly_apart(geo, pk, v2, rec_dist)) continue;
                     pwrap_dev(geo, pk, v2);
                     double d = len3_ref(rn_sub(pk[0], v2[0]), rn_sub(pk[1], v2[1]), rn_sub(pk[2], v2[2]));
                     if (d > rec_dist) continue;
@@ -406,6 +437,7 @@ __global__ void k_pairs(const uint64_t *__restrict__ keys, const int *__restrict
                     if (slot < pair_cap) { pairs[2 * slot] = k; pairs[2 * slot + 1] = l; }
                 }
             }
+        }
 }
 
 // remesh (tangle.c:1018-1061): the slots whose lengths could make the pass

@@ -232,3 +232,29 @@ def test_long_loop_smoothing_vs_oracle(detrend):
     ref = t.copy("pos")
     assert np.abs(out.pos - ref).max() < 1e-12
     assert np.abs(ref - pos0).max() > 1e-6   # it smoothed
+
+
+@pytest.mark.parametrize("images", ["periodic_26", "wall_2_4"])
+@pytest.mark.parametrize("cells", [1, 2, 3, 4, 40])
+def test_candidate_nodes_match_brute_force(cells, images):
+    """Nodes with another one within rec_dist (wrapped distance), for grids of one to
+    forty cells an axis: one range a row of cells, two where a row wraps."""
+    D = 0.1
+    ht = W.random_walk_tangle(6, 40, D=D, seed=cells)
+    ht = W.HostTangle(ht.pos.copy(), ht.conn[:, 0].copy(), ht.conn[:, 1].copy(), ht.box_lo, ht.box_hi,
+                      image_set=images)
+    rd = 0.499 * D / cells   # cells of 2 rec_dist
+    ctx = gpu.Context(0, params=W.config_params("rw", rec_dist=rd))
+    ctx.upload(ht)
+    ctx.update_tangle(0.0)
+    ctx.reconnect(0.0)
+    got = ctx.stats()["reconnect_candidates"]
+    ctx.close()
+    d = ht.pos[:, None, :] - ht.pos[None, :, :]
+    for a in range(3):
+        if ht.walls[2 * a] == abi.OV_WALL_PERIODIC:
+            d[..., a] -= D * np.rint(d[..., a] / D)
+    r = np.sqrt((d ** 2).sum(-1))
+    np.fill_diagonal(r, np.inf)
+    assert np.abs(r - rd).min() > 1e-12 * D, "a pair at the distance itself"
+    assert got == int((r.min(1) <= rd).sum())
