@@ -1874,15 +1874,24 @@ void ov_launch_tangents(ov_ctx *c, const NodeArrays &na, bool lia, cudaStream_t 
     c->launches++;
 }
 
-// Parts per query point: the FP64 split walk of a tangle too small to fill
-// the GPU with (tile, query group) items splits each walk into equal shares
-// of the pre-order cells (32 parts up to 2,048 slots, 8 up to 8,192), so a
-// kernel is not as long as its longest walk.
-constexpr int kSubWalkSlots = 8192;
-static int sub_walks_for(int cap) { return cap <= 2048 ? 32 : (cap <= kSubWalkSlots ? 8 : 1); }
-static int ov_sub_walks(const ov_ctx *c, int precision)
+// Parts per query point: where the FP64 split walk has few (tile, query group)
+// items for each SM, a walk is split into equal shares of the pre-order cells, so
+// that the launch does not end with a few warps in their last long walk.  Each part
+// pays its item's reads and the way down to its first cell, so not too many.
+// Traversal times (ms) with 1, 2, 4, 8, 16, 32 parts, by items an SM:
+//   496 nodes, 27 query points         3   .202 .150 .121 .098 .125 .190
+//   4,125 nodes, 19                   16  1.061 .778 .520 .399 .405 .481
+//   8,192 nodes, 27                   45   .907 .745 .573 .512 .649
+//   16,384 nodes, 27                  91  1.381 1.202 .953 1.107 1.366
+//   30,009 nodes, walls, 7            43  1.945 1.736 1.423 1.449
+//   32,768 nodes, 27                 182  2.125 1.912 1.925 2.288
+//   49,152 nodes, 27                 273  2.739 2.851 3.034 3.583
+constexpr int kItemsFor8 = 46, kItemsFor4 = 184;
+static int ov_sub_walks(ov_ctx *c, int precision)
 {
-    return ov_split_walk(c, precision) ? sub_walks_for(c->cap) : 1;
+    if (!ov_split_walk(c, precision)) return 1;
+    const long long items = (long long)((c->cap + 31) / 32) * ov_query_groups(c) / c->sm_count;
+    return items <= kItemsFor8 ? 8 : (items <= kItemsFor4 ? 4 : 1);
 }
 
 static bool has_mirror_images(const Geometry &g)
@@ -1930,7 +1939,7 @@ static int reserve_near_lists(ov_ctx *c, size_t warps)
 int ov_reserve_velocity_scratch(ov_ctx *c)
 {
     int G = ov_query_groups(c);
-    size_t need = (size_t)G * sub_walks_for(c->cap) * 6 * (size_t)c->cap;
+    size_t need = (size_t)G * ov_sub_walks(c, c->precision) * 6 * (size_t)c->cap;
     if (c->part_cap < need) {
         if (c->part) cudaFree(c->part);
         c->part = nullptr;

@@ -279,3 +279,20 @@ def test_rank_sorted_tree_is_the_radix_sorted_tree(n):
         got.append((np.array(ht.vs[:n]), [st[k] for k in ("cells", "max_depth", "visits", "accepts", "error_word")]))
     assert got[0][1] == got[1][1]
     np.testing.assert_array_equal(got[0][0], got[1][0])
+
+
+@pytest.mark.parametrize("loops,per_loop,images", [
+    (1, 5, "open"), (1, 33, "periodic_26"), (65, 127, "periodic_26"),   # 8 parts, fewer cells than parts, either side of 8 / 4
+    (70, 251, "wall_2_4"), (128, 255, "periodic_26"), (131, 256, "periodic_26")])   # 4 parts, either side of 4 / whole
+def test_parts_of_a_walk_add_up_to_the_whole_walk(loops, per_loop, images):
+    """The same cells visited and accepted as by the FP64 walk, which has no parts,
+    and the same velocities, at few and many (tile, query point) items an SM."""
+    base = W.random_walk_tangle(loops, per_loop, D=0.1, seed=12)
+    got = []
+    for walk in (abi.OV_WALK_FP64, abi.OV_WALK_SPLIT):
+        ht = W.HostTangle(base.pos.copy(), base.conn[:, 0].copy(), base.conn[:, 1].copy(), base.box_lo, base.box_hi,
+                          image_set=images)
+        st = _gpu_eval(ht, W.config_params("rw"), walk=walk)
+        got.append((np.array(ht.vels), [st[k] for k in ("visits", "accepts", "error_word")]))
+    assert got[0][1] == got[1][1] and got[0][1][2] == 0
+    assert node_rel_err(got[1][0], got[0][0]) < FP64_TOL
