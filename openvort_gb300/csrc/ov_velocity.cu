@@ -3605,6 +3605,8 @@ namespace {
 struct SphArgs {
     VelArgs v;                 // tree, positions, topology (slots [0, n) the tangle)
     int n;                     // slots of the tangle
+    int S;                     // parts per query point (split walk), else 1
+    double *pts;               // rotated query points, 8 x 3 arrays of n (split walk)
     double ri, ro;             // shell radii
     double d_az, d_pl;         // the section's full angular widths (rotation steps)
     double kappa, a0, alpha, alpha_p, dl_min, dl_max;
@@ -3869,53 +3871,84 @@ __global__ void __launch_bounds__(128) k_sph_query_mixed(SphArgs s, double *__re
     for (int ax = 0; ax < 3; ++ax) part[((size_t)q * 3 + ax) * s.n + id] = w[ax];
 }
 
+// Rotation steps of query point j = 0..7 of the 8 around the node itself.
+__device__ __forceinline__ void sph_step(const SphArgs &s, int j, double &da, double &dp)
+{
+    const double ua = j < 2 ? (j == 0 ? 1.0 : -1.0) : (j < 4 ? 0.0 : ((j & 1) ? -1.0 : 1.0));
+    const double up = j < 2 ? 0.0 : (j < 4 ? (j == 2 ? 1.0 : -1.0) : (j < 6 ? 1.0 : -1.0));
+    da = rn_mul(ua, s.d_az);
+    dp = rn_mul(up, s.d_pl);
+}
+
+// The rotated query points of every node, one thread each (the split walk's:
+// its parts and both members share them).
+__global__ void k_sph_points(SphArgs s)
+{
+    const int id = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y;
+    if (id >= s.n || s.v.status[id] == OV_EMPTY) return;
+    const double p[3] = {s.v.x[id], s.v.y[id], s.v.z[id]};
+    double da, dp, q[3];
+    sph_step(s, j, da, dp);
+    sph_rotate(p, da, dp, q);
+    for (int ax = 0; ax < 3; ++ax) s.pts[(size_t)(3 * j + ax) * s.n + id] = q[ax];
+}
+
 // k_sph_query on the FP64 path's split walk: the rotated query point split on
 // the grid for the FP32 tests (FP64 inside the guard bands), the accepted
-// cells evaluated in FP64 by the whole warp.
-__global__ void __launch_bounds__(128) k_sph_query_split(SphArgs s, double *__restrict__ part)
+// cells evaluated by the integer law.  Persistent warps take (query point, part,
+// tile) items: the walks differ in length, and with one warp of a fixed grid for
+// each the SMs were busy for 4.2 to 14.8 million cycles (16,000 nodes,
+// 7.15 ms; an evaluation 8.1 ms, 4.4 now).
+__global__ void __launch_bounds__(128, 4) k_sph_query_split(SphArgs s, double *__restrict__ part)
 {
     const VelArgs &a = s.v;
     const int lane = threadIdx.x & 31;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     WarpLists &lists = s_lists[threadIdx.x >> 5];
     const int nne = a.tt[TT_NNE];
     const int tiles = (nne + 31) / 32;
-    if (warp >= 18 * tiles) return;
-    const int q = warp / tiles, tile = warp - q * tiles;
-    const int loc = tile * 32 + lane;
-    bool valid = loc < nne;
-    int id = valid ? a.order[loc] : 0;
-    if (valid && (id < 0 || id >= s.n)) { bad_index(a, 9, id); valid = false; id = 0; }
-    const int st = valid ? a.status[id] : OV_EMPTY;
-    const bool take = valid && st != OV_PINNED && st != OV_EMPTY;
-    double p[3] = {0, 0, 0};
-    if (valid) { p[0] = a.x[id]; p[1] = a.y[id]; p[2] = a.z[id]; }
-    const int m = q / 9, j = q % 9 - 1;
-    const int root = a.tt[m * TT_WORDS + TT_ROOT], end = a.tt[m * TT_WORDS + TT_END];
-    const bool go = take && end > root;
-    double qp[3] = {p[0], p[1], p[2]}, da = 0, dp = 0;
-    if (j >= 0) {
-        const double ua = j < 2 ? (j == 0 ? 1.0 : -1.0) : (j < 4 ? 0.0 : ((j & 1) ? -1.0 : 1.0));
-        const double up = j < 2 ? 0.0 : (j < 4 ? (j == 2 ? 1.0 : -1.0) : (j < 6 ? 1.0 : -1.0));
-        da = rn_mul(ua, s.d_az);
-        dp = rn_mul(up, s.d_pl);
-        sph_rotate(p, da, dp, qp);
-    }
-    float g[3], f[3];
-    for (int ax = 0; ax < 3; ++ax) {
-        const double G = rint(qp[ax] * a.inv_h) * a.grid_h;
-        g[ax] = (float)G;
-        f[ax] = (float)(qp[ax] - G);
-    }
-    WalkCounts acc = {0u, 0u, 0u, 0u};
+    const int items = 18 * s.S * tiles;
+    unsigned long long vis = 0, ac = 0, fb = 0, steps = 0;
     bool overflow = false;
-    double v[3];
-    for (int ax = 0; ax < 3; ++ax) lists.q[ax][lane] = qp[ax];
-    walk_split(a, g, f, go ? 0 : 0x7fffffff, root, end, end, lists, lane, v, acc, overflow);
-    double w[3] = {v[0], v[1], v[2]};
-    if (j >= 0) sph_rotate(v, -da, -dp, w);
+    for (int it = next_item(a); it < items; it = next_item(a)) {
+        const int qs = it / tiles, tile = it - qs * tiles, q = qs / s.S, sub = qs - q * s.S;
+        const int loc = tile * 32 + lane;
+        bool valid = loc < nne;
+        int id = valid ? a.order[loc] : 0;
+        if (valid && (id < 0 || id >= s.n)) { bad_index(a, 9, id); valid = false; id = 0; }
+        const int st = valid ? a.status[id] : OV_EMPTY;
+        const bool take = valid && st != OV_PINNED && st != OV_EMPTY;
+        const int m = q / 9, j = q % 9 - 1;
+        const int root = a.tt[m * TT_WORDS + TT_ROOT], end = a.tt[m * TT_WORDS + TT_END];
+        const bool go = take && end > root;
+        float g[3], f[3];
+        const double *src[3] = {a.x, a.y, a.z};
+        __syncwarp();
+        for (int ax = 0; ax < 3; ++ax) {
+            double x = 0;
+            if (valid && st != OV_EMPTY) x = j < 0 ? src[ax][id] : s.pts[(size_t)(3 * j + ax) * s.n + id];
+            lists.q[ax][lane] = x;
+            const double G = rint(x * a.inv_h) * a.grid_h;
+            g[ax] = (float)G;
+            f[ax] = (float)(x - G);
+        }
+        __syncwarp();
+        // part `sub`: an equal share of the pre-order cells; the lane's state at
+        // its first cell from the walk down its ancestors
+        const long long nc = (long long)(end - root);
+        const int c0 = root + (int)(nc * sub / s.S), c1 = root + (int)(nc * (sub + 1) / s.S);
+        int resume0 = go ? 0 : 0x7fffffff;
+        if (go && c0 > root && c0 < c1) resume0 = ancestor_resume(a, root, end, c0, g, f, lists, lane);
+        WalkCounts acc = {0u, 0u, 0u, 0u};
+        double v[3];
+        walk_split(a, g, f, resume0, c0, end, c1, lists, lane, v, acc, overflow);
+        if (valid)
+            for (int ax = 0; ax < 3; ++ax) part[((size_t)(q * s.S + sub) * 3 + ax) * s.n + id] = v[ax];
+        vis += acc.nvis;
+        ac += acc.nacc;
+        fb += acc.nfb;
+        steps += acc.nstep;
+    }
     if (a.stat) {
-        unsigned long long vis = acc.nvis, ac = acc.nacc, fb = acc.nfb;
         for (int o = 16; o > 0; o >>= 1) {
             vis += __shfl_xor_sync(0xffffffffu, vis, o);
             ac += __shfl_xor_sync(0xffffffffu, ac, o);
@@ -3924,13 +3957,31 @@ __global__ void __launch_bounds__(128) k_sph_query_split(SphArgs s, double *__re
         if (lane == 0) {
             atomicAdd(&a.stat[ST_VISITS], vis);
             atomicAdd(&a.stat[ST_ACCEPTS], ac);
-            atomicAdd(&a.stat[ST_STEPS], (unsigned long long)acc.nstep);
+            atomicAdd(&a.stat[ST_STEPS], steps);
             atomicAdd(&a.stat[ST_FALLBACK], fb);
         }
     }
     if (overflow && lane == 0) atomicOr((int *)&a.counters[TC_ERR], OV_EW_ITER);
-    if (!valid) return;
-    for (int ax = 0; ax < 3; ++ax) part[((size_t)q * 3 + ax) * s.n + id] = w[ax];
+}
+
+// A query point's parts added in part order and turned back, into the first
+// part's place: one thread per node and query point.
+__global__ void k_sph_sum(SphArgs s, double *__restrict__ part)
+{
+    const int id = blockIdx.x * blockDim.x + threadIdx.x, q = blockIdx.y;
+    if (id >= s.n || s.v.status[id] == OV_EMPTY) return;
+    double v[3] = {0, 0, 0}, w[3];
+    for (int k = 0; k < s.S; ++k)
+        for (int ax = 0; ax < 3; ++ax) v[ax] += part[((size_t)(q * s.S + k) * 3 + ax) * s.n + id];
+    const int j = q % 9 - 1;
+    if (j >= 0) {
+        double da, dp;
+        sph_step(s, j, da, dp);
+        sph_rotate(v, -da, -dp, w);
+    } else {
+        for (int ax = 0; ax < 3; ++ax) w[ax] = v[ax];
+    }
+    for (int ax = 0; ax < 3; ++ax) part[((size_t)(q * s.S) * 3 + ax) * s.n + id] = w[ax];
 }
 
 // The rest of update_velocity (tangle.c:644-665, 763-865 of the fork): the
@@ -3948,7 +3999,7 @@ __global__ void k_sph_finish(SphArgs s, const double *__restrict__ part)
         return;
     }
     const double p[3] = {a.x[id], a.y[id], a.z[id]};
-    auto P = [&](int q, int ax) { return part[((size_t)q * 3 + ax) * s.n + id]; };
+    auto P = [&](int q, int ax) { return part[((size_t)(q * s.S) * 3 + ax) * s.n + id]; };
     double own[3], tot[3] = {0, 0, 0};
     for (int ax = 0; ax < 3; ++ax) own[ax] = P(0, ax);
     for (int q = 1; q < 9; ++q)
@@ -4023,6 +4074,8 @@ SphArgs make_sph_args(ov_ctx *c, const SphDomain &d, const SphSettings &p)
     s.v = make_args(c, c->node, 0.0, ov_stat_ptr(c));
     s.v.tid = nullptr; s.v.tprm = nullptr; s.v.mrange = nullptr; s.v.qorder = nullptr;
     s.n = d.n;
+    s.S = 1;
+    s.pts = nullptr;
     s.ri = d.ri; s.ro = d.ro;
     s.d_az = 2 * d.az; s.d_pl = 2 * d.pl;
     s.kappa = p.kappa; s.a0 = p.a0; s.alpha = p.alpha; s.alpha_p = p.alpha_p;
@@ -4050,10 +4103,18 @@ void ov_launch_sph_images(ov_ctx *c, const SphDomain &d, const SphSettings &p)
     c->launches++;
 }
 
+constexpr int kSphItemsFor8 = 768;   // (tile, query point) items an SM
 int ov_launch_sph_velocities(ov_ctx *c, const SphDomain &d, const SphSettings &p)
 {
     SphArgs s = make_sph_args(c, d, p);
-    const size_t need = (size_t)18 * 3 * (size_t)d.n;
+    // Parts of the split walk, whose lengths differ more than a box's (1, 4, 8 parts:
+    // 4,000 nodes 3.2, 1.6, 1.4 ms an evaluation, 16,000 8.4, 4.7, 4.4, 55,000 19.4, 17.1,
+    // 16.5, 187,500 68.4, 64.8, 63.6), and its rotated points behind them.  Beyond that
+    // the parts' room (3.5 kB a node) is not worth the few percent.
+    const bool split = c->precision != OV_PREC_MIXED && c->walk == OV_WALK_SPLIT;
+    const long long per_sm = 18LL * ((d.n + 31) / 32) / c->sm_count;
+    s.S = split && per_sm <= kSphItemsFor8 ? 8 : 1;
+    const size_t need = (size_t)(18 * s.S + (split ? 8 : 0)) * 3 * (size_t)d.n;
     if (c->part_cap < need) {
         if (c->part) cudaFree(c->part);
         c->part = nullptr;
@@ -4063,9 +4124,16 @@ int ov_launch_sph_velocities(ov_ctx *c, const SphDomain &d, const SphSettings &p
     const long long warps = 18LL * ((d.n + 31) / 32);
     if (c->precision == OV_PREC_MIXED)
         k_sph_query_mixed<<<(unsigned)((warps + 3) / 4), 128, 0, c->stream>>>(s, c->part);
-    else if (c->walk == OV_WALK_SPLIT)
-        k_sph_query_split<<<(unsigned)((warps + 3) / 4), 128, 4 * sizeof(WarpLists), c->stream>>>(s, c->part);
-    else
+    else if (split) {
+        s.pts = c->part + (size_t)18 * s.S * 3 * d.n;
+        const unsigned blocks = (unsigned)std::min((warps * s.S + 3) / 4, 4LL * c->sm_count);   // 4 blocks an SM
+        const unsigned rows = (unsigned)((d.n + 127) / 128);
+        OV_CUDA(c, cudaMemsetAsync(s.v.work, 0, sizeof(int), c->stream));
+        k_sph_points<<<dim3(rows, 8), 128, 0, c->stream>>>(s);
+        k_sph_query_split<<<std::max(blocks, 1u), 128, 4 * sizeof(WarpLists), c->stream>>>(s, c->part);
+        k_sph_sum<<<dim3(rows, 18), 128, 0, c->stream>>>(s, c->part);
+        c->launches += 2;
+    } else
         k_sph_query<<<(unsigned)((warps + 3) / 4), 128, 0, c->stream>>>(s, c->part);
     k_sph_finish<<<(d.n + 127) / 128, 128, 0, c->stream>>>(s, c->part);
     c->launches += 2;
