@@ -1,12 +1,18 @@
 // ov_velocity.cu - per-node velocity kernels.
 //
-//  k_tangents     update_tangent_normal (tangle.c:423-502), one node per thread
-//  k_vel_fp64     update_velocity (tangle.c:600-726) fused: LIA + external
-//                 v_s + Barnes-Hut over the primary and every image query
-//                 point + mutual friction, one warp per 32 Morton-ordered
-//                 targets sharing one cursor through the pre-order cells
-//  k_rec_sums     direct sums, the tree==NULL branch (tangle.c:652-687), in
+//  k_tangents     update_tangent_normal (tangle.c:423-502) and the local (LIA) velocity,
+//                 one node per thread
+//  k_vel_split    update_velocity's Barnes-Hut sums, the default FP64 path: FP32 tests,
+//                 interactions on 64-bit integer mantissas (ov_fxlaw.cuh)
+//  k_vel_fp64     update_velocity (tangle.c:600-726), every test in FP64:
+//                 Barnes-Hut over the primary and every image query
+//                 point, one warp per 32 Morton-ordered targets sharing one
+//                 cursor through the pre-order cells
+//  k_vel_finish   the sums, external v_s and mutual friction
+//  k_direct_fx    direct sums, the tree==NULL branch (tangle.c:652-687), in
 //                 (node, segment chunk) blocks; k_direct_finish adds LIA etc.
+//  k_rec_far      reconnection candidates' direct sums by a far-segment series with an
+//                 error bound; k_rec_sums where images mirror, and the refinements
 //  k_euler / k_rk4_combine / k_wrap   RK4 stages and enforce_periodic_boundaries
 //
 // The FP64 traversal keeps the reference's decisions bit-for-bit given the
