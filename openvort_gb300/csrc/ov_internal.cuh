@@ -18,7 +18,9 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <math.h>
 #include <stdint.h>
+#include <algorithm>
 #include <string>
 #include <vector>
 
@@ -367,8 +369,11 @@ inline bool ov_split_walk(const ov_ctx *c, int precision)
 }
 // Unit of the integer law's coordinates: grid step / 2^bits, every separation
 // below 2^61 units (a box's grid leaves two periods of room, a spherical
-// section's none).
-inline int ov_fx_bits(const ov_ctx *c) { return c->geo.sph ? 38 : 39; }
+// section's none).  Not below 2^-75: what the law takes is then at least 2^51
+// units = 6e-8 away at one end and a quarter of that at the other, where the
+// reference's filters (|R|, |R+S| < 1e-8) drop nothing; closer cells of boxes
+// smaller than 2e-5 are left to the FP64 law, which has the filters.
+inline double ov_fx_inv(const ov_ctx *c) { return std::min(ldexp(1.0 / c->grid_h, c->geo.sph ? 38 : 39), 0x1p75); }
 
 // sort / scan (ov_sort.cu)
 void ov_sort_keys(ov_ctx *c, TreeBuf &t, int n, cudaStream_t s);

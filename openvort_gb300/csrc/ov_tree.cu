@@ -1067,7 +1067,7 @@ int ov_tree_build(ov_ctx *c, const NodeArrays &na, cudaStream_t s)
     const bool fp32_view = c->precision == OV_PREC_MIXED || c->precision == OV_PREC_DD || c->walk == OV_WALK_SPLIT;
     views.c32 = fp32_view ? t.cells32 : nullptr;
     views.cfx = ov_split_walk(c, c->precision) ? t.cellsfx : nullptr;
-    views.fx_inv = ldexp(1.0 / c->grid_h, ov_fx_bits(c));
+    views.fx_inv = ov_fx_inv(c);
     views.h = c->grid_h;
     views.inv_h = 1.0 / c->grid_h;
     views.theta = c->params.bh_resolution;

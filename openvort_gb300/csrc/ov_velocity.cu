@@ -1815,7 +1815,7 @@ VelArgs make_args(ov_ctx *c, const NodeArrays &na, double t, unsigned long long 
     a.cells = c->tree.cells;
     a.cells32 = c->tree.cells32;
     a.cellsfx = c->tree.cellsfx;
-    a.fx_inv = c->grid_h > 0 ? ldexp(1.0 / c->grid_h, ov_fx_bits(c)) : 0;
+    a.fx_inv = c->grid_h > 0 ? ov_fx_inv(c) : 0;
     a.x = na.x; a.y = na.y; a.z = na.z;
     a.tx = na.tx; a.ty = na.ty; a.tz = na.tz;
     a.nx = na.nx; a.ny = na.ny; a.nz = na.nz;
@@ -3210,7 +3210,7 @@ int rec_launch_fx(ov_ctx *c, const RecArgs &ra, const int *d_nodes, int n, int *
         OV_ALLOC(c, cudaMalloc(&c->rec_seg, (size_t)c->cap * sizeof(CellFX)));
         c->rec_seg_cap = c->cap;
     }
-    const double fx_inv = ldexp(1.0 / c->grid_h, ov_fx_bits(c));
+    const double fx_inv = ov_fx_inv(c);
     k_segments_fx<<<(c->cap + 255) / 256, 256, 0, c->stream>>>(ra, fx_inv, c->rec_seg);
     k_direct_fx<<<dim3(n, *chunks), kRecThreads, 0, c->stream>>>(ra, fx_inv, c->rec_seg, d_nodes, n, span, *chunks,
                                                                 c->rec_part);
