@@ -587,6 +587,7 @@ static void set_geometry(ov_ctx *c, const ov_domain_box &box, const ov_boundary_
     for (int a = 0; a < 3; ++a) m = std::max(m, std::max(fabs(g.lo[a]), fabs(g.hi[a])) + 2 * fabs(g.L[a]));
     int e = (int)ceil(log2(m > 0 ? m : 1.0));
     c->grid_h = ldexp(1.0, e - 22);
+    c->fx = fx_frame(g.lo, g.hi);
 }
 
 // Per-member device tables: build table, parameters, queue order, slot
@@ -1461,7 +1462,9 @@ static int sph_run(ov_ctx *c, ov_sph_tangle_state *t, const ov_sph_params *p, do
     g.sph_pl = dom.polar_angle;
     g.sph_seg_max = 5 * p->dl_max;
     // grid step of the mixed path: every coordinate (|x| <= ro) below 2^22 steps
-    c->grid_h = ldexp(1.0, (int)ceil(log2(dom.outer_radius)) - 22);
+    const int ero = (int)ceil(log2(dom.outer_radius));
+    c->grid_h = ldexp(1.0, ero - 22);
+    c->fx = fx_unit(ero - 60);   // every coordinate below 2^60 units, every separation below 2^61
     const double A = dom.azimut_angle, P = dom.polar_angle;
     const double ri = dom.inner_radius, ro = dom.outer_radius;
     const double lo0[3] = {ri, -A, -P}, hi0[3] = {ro, A, P};

@@ -7,8 +7,8 @@
 // and 1.8 lanes a cycle and SM for IMAD.WIDE, IADD and DFMA).  The law
 // (octree.c:321-342)
 //     w = (R x S) (|R| + |R+S|) / (|R||R+S| (|R||R+S| + R.(R+S)))
-// therefore runs on fixed-point coordinates (unit u = grid step / 2^39, every
-// separation below 2^61 units, so positions of FP64 magnitude down to 2^-9 of
+// therefore runs on fixed-point coordinates (FxFrame: counted from the box, every
+// separation below 2^61 units u, so offsets of FP64 magnitude down to 2^-9 of
 // the largest convert exactly), left-normalised per interaction, with 2 to 9
 // IMAD.WIDE per product.  Each of the two square roots and the quotient
 // starts from the FP32 hardware approximation and takes two exact integer
@@ -17,8 +17,9 @@
 // cancels by |R| / |S|; the terms add up exactly, in 96 bits.
 //
 // What this cannot decide or would lose bits on is left to the FP64 law:
-// interactions nearer than 2^12 grid steps, ends at distances that differ
-// fourfold, or seen almost 90 degrees or more apart (where the reference's
+// interactions nearer than 2^47 units (a 2,000th to a 5,500th of a cubic box's side,
+// wherever the box lies; 2^51 where coordinates had to be rounded), ends at
+// distances that differ fourfold, or seen almost 90 degrees or more apart (where the reference's
 // ndot filter drops them).
 //
 // Host and device: the arithmetic is integer apart from the FP32 seeds, whose
@@ -28,27 +29,77 @@
 
 #include <math.h>
 #include <stdint.h>
+#include <string.h>
 
 // FP64 cell view of the integer law (64 bytes).  c: centre of mass in units
 // u; s: circulation in units u, shifted left by e so that its largest
 // component is in [2^60, 2^61), as sh 2^32 + sl; n: |s|^2 / 2^64.
 // e = kFxNone: not representable (FP64 law); e = kFxZero: zero circulation
-// (no velocity).
+// (no velocity).  shift: separations below 2^(60 - shift) units are left to the
+// FP64 law.
 struct alignas(16) CellFX {
     int64_t c[3];
     int sh[3], sl[3];
     int64_t n;
-    int e, pad;
+    int e, shift;
 };
 constexpr int kFxNone = -1, kFxZero = -2;
-constexpr int kFxMaxShift = 9;     // |R| below 2^(60 - 9) units: FP64 law
+// Largest shift: kFxMaxShift keeps a coordinate's rounding to a unit below 2^-52 of
+// the separation; where both sides are whole numbers of units without rounding
+// (most of a box: all but its 512th next to the planes from which it is counted) the
+// separation is exact, and kFxWholeShift is where terms pass 2^58 units of the sums;
+// kFxRoundShift does for coordinates that lose bits when they are counted from
+// the box's corner (2^7 units at most: points far outside the box toward 0)
+// (65,536 nodes in a 200th of their open box: traversal 10.9 ms with 9 throughout, late
+// cells evaluated one by one where their list was full; 6.8 with 9 and the list flushed,
+// 4.8 with 13).
+constexpr int kFxMaxShift = 9, kFxWholeShift = 13, kFxRoundShift = 2;
 // Terms add up in units 2^kFxUnit / u.  A term's error is about 2^-8 units (the
 // aligned quotient's last bit), and terms with a quotient above 2^63 units, the
 // nearest, are left to the FP64 law: the unit of a tree's sums (2,000 terms)
 // sends it a handful, that of direct sums (10^6 terms) a few hundred.
 constexpr int kFxUnit = -105, kFxUnitDirect = -110;
 constexpr int kFxTerms = 31;       // terms a sum holds: each is at most 2^58 units
-constexpr double kFxLimit = 2305843009213693952.0;   // 2^61: coordinates a view holds
+constexpr double kFxLimit = 2305843009213693952.0;   // 2^61: coordinates are below
+
+// Fixed-point coordinates: x in units u is x inv + at, u = 1 / inv.
+struct FxFrame {
+    double inv, u, at[3];
+    int e;       // inv = 2^e
+    int whole;   // largest shift of whole coordinates
+};
+static inline FxFrame fx_unit(int e)   // unit 2^e, counted from 0
+{
+    // Not below 2^-75, and the shift so that what the law takes is at least 2^-24 =
+    // 6e-8 away at one end and a quarter of that at the other, where the reference's
+    // filters (|R|, |R+S| < 1e-8) drop nothing: closer cells, of boxes smaller than
+    // 3e-4, are left to the FP64 law, which has the filters.
+    if (e < -75) e = -75;
+    const int s = 60 + 24 + e;
+    return FxFrame{ldexp(1.0, -e), ldexp(1.0, e), {0, 0, 0}, -e, s < kFxWholeShift ? s : kFxWholeShift};
+}
+
+// The frame of a box: counted from 0 where the box is within its length of it,
+// else from the corner nearest to 0 rounded to 2^-22 of the box (coordinates of the
+// box then lose nothing), so that the unit depends on the box's lengths; it leaves
+// a period on either side (image query points, stage positions) below 2^61 units.
+// (A unit taken from the largest coordinate leaves most interactions of a box far
+// from 0 to the FP64 law: 65,536 nodes in a box of side 0.1, traversal 3.6 ms at 0,
+// 9.6 at 10 and 17.2 at 50; 3.7 wherever it lies so.)
+static inline FxFrame fx_frame(const double lo[3], const double hi[3])
+{
+    FxFrame f;
+    double o[3], L = 0, m = 0;
+    for (int a = 0; a < 3; ++a) L = fmax(L, fabs(hi[a] - lo[a]));
+    const double step = ldexp(1.0, (int)ceil(log2(L > 0 ? L : 1.0)) - 22);
+    for (int a = 0; a < 3; ++a) {
+        o[a] = lo[a] > L ? floor(lo[a] / step) * step : (hi[a] < -L ? ceil(hi[a] / step) * step : 0.0);
+        m = fmax(m, fmax(fabs(lo[a] - o[a]), fabs(hi[a] - o[a])) + 2 * fabs(hi[a] - lo[a]));
+    }
+    f = fx_unit((int)ceil(log2(m > 0 ? m : 1.0)) - 61);
+    for (int a = 0; a < 3; ++a) f.at[a] = -o[a] * f.inv;
+    return f;
+}
 
 #if defined(__CUDA_ARCH__)
 #define FX_INLINE __device__ __forceinline__
@@ -81,6 +132,40 @@ FX_INLINE int64_t fx_shr(int64_t x, int n) { return x >> (n < 63 ? n : 63); }
 FX_INLINE int64_t fx_mad(int a, int b, int64_t c) { return c + (int64_t)a * b; }
 FX_INLINE uint64_t fx_madu(unsigned a, unsigned b, uint64_t c) { return c + (uint64_t)a * b; }
 #endif
+
+FX_INLINE uint64_t fx_bits(double x)
+{
+#if defined(__CUDA_ARCH__)
+    return (uint64_t)__double_as_longlong(x);
+#else
+    uint64_t b;
+    memcpy(&b, &x, 8);
+    return b;
+#endif
+}
+
+// x is a whole number: no bits of its fraction below 1
+FX_INLINE bool fx_whole(double x)
+{
+    const uint64_t b = fx_bits(x);
+#if defined(__CUDA_ARCH__)
+    const int low = __ffsll((long long)(b | (1ull << 52))) - 1;
+#else
+    const int low = __builtin_ctzll(b | (1ull << 52));
+#endif
+    return (int)((b >> 52) & 0x7ff) - 1023 + low >= 52 || b << 1 == 0;
+}
+
+// Largest shift that a coordinate r = x inv + at allows, -1: 2^61 or more, or no
+// number.  r is a multiple of x's last bit, so it was rounded only if it is of a
+// larger magnitude than x inv.
+FX_INLINE int fx_shift(double r, double x, const FxFrame &f)
+{
+    const int er = (int)((fx_bits(r) >> 52) & 0x7ff), ex = (int)((fx_bits(x) >> 52) & 0x7ff);
+    if (er >= 1023 + 61) return -1;
+    if (er != 0 && er - ex > f.e) return kFxRoundShift;
+    return fx_whole(r) ? f.whole : kFxMaxShift;
+}
 
 FX_INLINE int fx_hi(int64_t x) { return (int)(x >> 32); }
 FX_INLINE int64_t fx_mul(int a, int b) { return (int64_t)a * b; }
@@ -141,7 +226,7 @@ FX_INLINE int64_t fx_mulhi(int64_t a, int64_t b)
 
 // The view of a cell or segment from its coordinates in units u; fits: they
 // are below 2^61.
-FX_INLINE CellFX fx_cell(const int64_t c[3], const int64_t s[3], bool fits)
+FX_INLINE CellFX fx_cell(const int64_t c[3], const int64_t s[3], bool fits, int shift = kFxMaxShift)
 {
     CellFX o;
     uint64_t m = 0;
@@ -159,16 +244,17 @@ FX_INLINE CellFX fx_cell(const int64_t c[3], const int64_t s[3], bool fits)
         low = fx_mad(p.h, p.l, low);
     }
     o.n += low >> 31;
-    o.pad = 0;
+    o.shift = shift;
     return o;
 }
 
 // Adds the law's term for cell c seen from q (units u) to sum where `take` is
 // set and the law can decide; returns that (no branches: what is left to the
-// FP64 law is rare).  mag, when given, gains a bound on the term's
+// FP64 law is rare).  shift: the largest that q allows.  mag, when given, gains a bound on the term's
 // magnitude (over the components, in the sum's units, to FP32 precision).
 template <int Unit = kFxUnit>
-FX_INLINE bool fx_law(const CellFX &c, const int64_t q[3], bool take, fx_sum sum[3], float *mag = nullptr)
+FX_INLINE bool fx_law(const CellFX &c, const int64_t q[3], bool take, fx_sum sum[3], int shift = kFxMaxShift,
+                      float *mag = nullptr)
 {
     int64_t R[3];
     unsigned top = 0;
@@ -178,7 +264,7 @@ FX_INLINE bool fx_law(const CellFX &c, const int64_t q[3], bool take, fx_sum sum
         top |= (unsigned)(h ^ (h >> 31));
     }
     const int sr = fx_clz(top) - 3;
-    bool ok = take && (unsigned)sr <= (unsigned)kFxMaxShift && c.e >= 0;
+    bool ok = take && (unsigned)sr <= (unsigned)(shift < c.shift ? shift : c.shift) && c.e >= 0;
     const int s = (sr < c.e ? sr : c.e) & 63, ds = (c.e - s) & 63;
     // a = |R|^2, m = R.S, both / 2^64
     fx_split r[3];

@@ -26,6 +26,7 @@
 
 #include "../../include/openvort_gpu.h"
 #include "../../include/ov_spherical.h"
+#include "ov_fxlaw.cuh"
 
 #define OV_MAX_LEVEL 21                 // 3-bit digits below the root: 63 bits
 #define OV_KEY_OUT (0x8000000000000000ull) // node outside the root box (| wrapped path >> 1)
@@ -77,8 +78,6 @@ enum MemberWords {
 
 constexpr int TREE_LV_SLOTS = 32;   // levels 0..OV_MAX_LEVEL of the per-level cell lists
 constexpr int TREE_INV_COUNT = 4096; // table of 1 / count for the cell means
-
-struct CellFX;             // 64 bytes: fixed-point view for the FP64 path (ov_fxlaw.cuh)
 
 struct TreeBuf {
     int cap = 0;
@@ -267,6 +266,7 @@ struct ov_ctx {
     int64_t rk4_kernels = 0;     // kernels in the captured RK4 graph
     // mixed-precision grid split
     double grid_h = 0;
+    FxFrame fx = {};             // fixed-point coordinates of the integer law
     // per-group partial velocity sums of the traversal (6 doubles x groups x cap)
     double *part = nullptr;
     size_t part_cap = 0;
@@ -367,13 +367,6 @@ inline bool ov_split_walk(const ov_ctx *c, int precision)
 {
     return precision == OV_PREC_DD || (precision == OV_PREC_FP64 && c->walk == OV_WALK_SPLIT);
 }
-// Unit of the integer law's coordinates: grid step / 2^bits, every separation
-// below 2^61 units (a box's grid leaves two periods of room, a spherical
-// section's none).  Not below 2^-75: what the law takes is then at least 2^51
-// units = 6e-8 away at one end and a quarter of that at the other, where the
-// reference's filters (|R|, |R+S| < 1e-8) drop nothing; closer cells of boxes
-// smaller than 2e-5 are left to the FP64 law, which has the filters.
-inline double ov_fx_inv(const ov_ctx *c) { return std::min(ldexp(1.0 / c->grid_h, c->geo.sph ? 38 : 39), 0x1p75); }
 
 // sort / scan (ov_sort.cu)
 void ov_sort_keys(ov_ctx *c, TreeBuf &t, int n, cudaStream_t s);

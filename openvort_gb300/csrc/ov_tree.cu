@@ -23,7 +23,6 @@
 // is empty and the keys hold 21 levels; with T members it takes
 // ceil(log2 T) bits and the keys hold floor((63 - bits) / 3) levels.
 #include "ov_internal.cuh"
-#include "ov_fxlaw.cuh"
 
 void ov_sort_keys(ov_ctx *c, TreeBuf &t, int n, cudaStream_t s);
 int ov_sort_hist_ints(int cap);
@@ -428,18 +427,20 @@ __device__ __forceinline__ void write_cell32(Cell32 *out, int ci, const double c
 }
 
 // Fixed-point view for the FP64 path's integer law (ov_fxlaw.cuh): centre of
-// mass and circulation in units 1 / fx_inv, the circulation left-normalised.
-__device__ __forceinline__ void write_cellfx(CellFX *out, int ci, const double c[3], const double q[3], double fx_inv)
+// mass and circulation in the frame's units, the circulation left-normalised.
+__device__ __forceinline__ void write_cellfx(CellFX *out, int ci, const double c[3], const double q[3],
+                                             const FxFrame &fx)
 {
-    bool fits = true;
+    int shift = fx.whole;
     int64_t x[3], s[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        fits = fits && fabs(c[a] * fx_inv) < kFxLimit && fabs(q[a] * fx_inv) < kFxLimit;
-        x[a] = __double2ll_rn(c[a] * fx_inv);
-        s[a] = __double2ll_rn(q[a] * fx_inv);
+        const double cu = fma(c[a], fx.inv, fx.at[a]), qu = q[a] * fx.inv;
+        shift = min(min(shift, fx_shift(cu, c[a], fx)), fx_shift(qu, q[a], fx));
+        x[a] = __double2ll_rn(cu);
+        s[a] = __double2ll_rn(qu);
     }
-    const CellFX o = fx_cell(x, s, fits);
+    const CellFX o = fx_cell(x, s, shift >= 0, shift);
     const int4 *src = reinterpret_cast<const int4 *>(&o);
     int4 *dst = reinterpret_cast<int4 *>(out + ci);
 #pragma unroll
@@ -451,7 +452,7 @@ __device__ __forceinline__ void write_cellfx(CellFX *out, int ci, const double c
 struct CellViews {
     Cell32 *c32;
     CellFX *cfx;
-    double fx_inv;
+    FxFrame fx;
     double h, inv_h, theta;
     const double *inv_count;   // 1 / k for k < TREE_INV_COUNT
     const float *lev_tab;      // box cells: threshold and Lm per level (null: spherical cells)
@@ -481,7 +482,7 @@ __device__ __forceinline__ void store_cell(Cell64 *cells, int ci, const double s
         const float lm32 = v.lev_tab ? v.lev_tab[TREE_LV_SLOTS + lev] : __double2float_ru(lm);
         write_cell32(v.c32, ci, c, q, thr, lm32, next, v.h, v.inv_h);
     }
-    if (v.cfx) write_cellfx(v.cfx, ci, c, q, v.fx_inv);
+    if (v.cfx) write_cellfx(v.cfx, ci, c, q, v.fx);
 }
 
 __device__ __forceinline__ void store_psum(double *psum, int ci, const double acc[6])
@@ -797,9 +798,13 @@ __device__ __forceinline__ void lane_store(bool ok, int k, int ci, const LaneSum
         else if (ok && k == 6) { o[3] = thr; o[7] = __int_as_float(r.next); o[11] = lm32; }
     }
     if (v.cfx) {
-        const bool in = k >= 6 || fabs(c * v.fx_inv) < kFxLimit;
-        const int64_t w = __double2ll_rn(c * v.fx_inv);
-        const unsigned m = __ballot_sync(0xffffffffu, in);
+        const double at = k == 0 ? v.fx.at[0] : (k == 1 ? v.fx.at[1] : (k == 2 ? v.fx.at[2] : 0.0));
+        const double cu = fma(c, v.fx.inv, at);
+        const int64_t w = __double2ll_rn(cu);
+        const int mine = k < 6 ? fx_shift(cu, c, v.fx) : v.fx.whole;   // the group's: the least
+        const unsigned low = __ballot_sync(0xffffffffu, mine < v.fx.whole);
+        const unsigned least = __ballot_sync(0xffffffffu, mine == kFxRoundShift);
+        const unsigned out = __ballot_sync(0xffffffffu, mine < 0);
         const int g8 = threadIdx.x & 24;
         int64_t x[3], q[3];
 #pragma unroll
@@ -808,7 +813,8 @@ __device__ __forceinline__ void lane_store(bool ok, int k, int ci, const LaneSum
             q[a] = __shfl_sync(0xffffffffu, w, g8 + 3 + a);
         }
         if (ok && k == 0) {
-            const CellFX o = fx_cell(x, q, ((m >> g8) & 63u) == 63u);
+            const int shift = (least >> g8) & 63u ? kFxRoundShift : ((low >> g8) & 63u ? kFxMaxShift : v.fx.whole);
+            const CellFX o = fx_cell(x, q, ((out >> g8) & 63u) == 0, shift);
             const int4 *src = reinterpret_cast<const int4 *>(&o);
             int4 *dst = reinterpret_cast<int4 *>(v.cfx + ci);
 #pragma unroll
@@ -1067,7 +1073,7 @@ int ov_tree_build(ov_ctx *c, const NodeArrays &na, cudaStream_t s)
     const bool fp32_view = c->precision == OV_PREC_MIXED || c->precision == OV_PREC_DD || c->walk == OV_WALK_SPLIT;
     views.c32 = fp32_view ? t.cells32 : nullptr;
     views.cfx = ov_split_walk(c, c->precision) ? t.cellsfx : nullptr;
-    views.fx_inv = ov_fx_inv(c);
+    views.fx = c->fx;
     views.h = c->grid_h;
     views.inv_h = 1.0 / c->grid_h;
     views.theta = c->params.bh_resolution;

@@ -25,7 +25,6 @@
 #include <algorithm>
 
 #include "ov_internal.cuh"
-#include "ov_fxlaw.cuh"
 
 #ifndef M_PI
 #define M_PI 3.14159265358979323846
@@ -53,7 +52,7 @@ struct VelArgs {
     const Cell64 *cells;
     const Cell32 *cells32;
     const CellFX *cellsfx;      // split walk: fixed-point cell data
-    double fx_inv;              // 1 / its unit (a power of two)
+    FxFrame fx;                 // its coordinates
     const double *x, *y, *z, *tx, *ty, *tz, *nx, *ny, *nz;
     double *vx, *vy, *vz, *sx, *sy, *sz;
     const int *fwd, *rev, *status, *pin;
@@ -1481,21 +1480,32 @@ __device__ __forceinline__ CellFX load_cellfx(const CellFX *p)
     return c;
 }
 
+// Largest shift of the integer law that the lane's query point allows, -1: the point
+// is out of its range.
+__device__ __forceinline__ int query_shift(const FxFrame &fx)
+{
+    const int lane = threadIdx.x & 31;
+    const WarpLists &L = s_lists[threadIdx.x >> 5];
+    int shift = fx.whole;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const double p = L.q[i][lane];
+        shift = min(shift, fx_shift(fma(p, fx.inv, fx.at[i]), p, fx));
+    }
+    return shift;
+}
+
 // Evaluate the last min(n, rows) entries of every lane's list at its query
 // point; the sum in units kappa / 4 pi / u.  Cells left to the FP64 law go to
 // the late list (or are evaluated when it is full).
-__device__ __forceinline__ double3 run_list(const CellFX *cells, const Cell64 *cells64, int rows, int n, double fx_inv)
+__device__ __forceinline__ double3 run_list(const CellFX *cells, const Cell64 *cells64, int rows, int n, int shift,
+                                            const FxFrame &fx)
 {
     const int lane = threadIdx.x & 31;
     WarpLists &L = s_lists[threadIdx.x >> 5];
     int64_t q[3];
-    bool in_range = true;
 #pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        const double x = L.q[i][lane] * fx_inv;
-        in_range = in_range && fabs(x) < kFxLimit;
-        q[i] = __double2ll_rn(x);
-    }
+    for (int i = 0; i < 3; ++i) q[i] = __double2ll_rn(fma(L.q[i][lane], fx.inv, fx.at[i]));
     double v[3] = {0.0, 0.0, 0.0};
     const double unit = ldexp(1.0, kFxUnit);
     while (rows > 0) {
@@ -1506,7 +1516,7 @@ __device__ __forceinline__ double3 run_list(const CellFX *cells, const Cell64 *c
             if (n == 0) continue;
             const int cell = L.entry[32 * --n + lane];
             const CellFX c = load_cellfx(cells + cell);
-            if (!fx_law(c, q, in_range, sum) && !(in_range && c.e == kFxZero)) {
+            if (!fx_law(c, q, shift >= 0, sum, shift) && !(shift >= 0 && c.e == kFxZero)) {
                 const int late = L.nlate[lane];
                 if (late < kLateCap) {
                     L.late[32 * late + lane] = cell;
@@ -1515,7 +1525,7 @@ __device__ __forceinline__ double3 run_list(const CellFX *cells, const Cell64 *c
                     const double qd[3] = {L.q[0][lane], L.q[1][lane], L.q[2][lane]};
                     double w[3];
                     law64_term(cells64 + cell, qd, w);
-                    for (int i = 0; i < 3; ++i) v[i] += w[i] / fx_inv;
+                    for (int i = 0; i < 3; ++i) v[i] = fma(w[i], fx.u, v[i]);
                 }
             }
         }
@@ -1619,6 +1629,7 @@ __device__ __forceinline__ void walk_split(const VelArgs &a, const float g[3], c
 {
     v[0] = v[1] = v[2] = 0.0;
     L.nlate[lane] = 0;
+    const int shift = query_shift(a.fx);
     const float2 ng01 = make_float2(-g[0], -g[1]), nf01 = make_float2(-f[0], -f[1]);
     int c = root;
     int resume = resume0;
@@ -1649,16 +1660,22 @@ __device__ __forceinline__ void walk_split(const VelArgs &a, const float g[3], c
         ++steps;
         // a lane adds at most one entry a step: room for kListStep more after this test
         if ((steps & (kListStep - 1)) == 0 && __any_sync(0xffffffffu, n > kListCap - kListStep)) {
-            const double3 w = run_list(a.cellsfx, a.cells, kListCap / 2, n, a.fx_inv);
+            // room for late cells, of which a run of the list may add many
+            const int late = __reduce_max_sync(0xffffffffu, L.nlate[lane]);
+            if (late > kLateCap / 2) {
+                const double3 w = run_late(a.cells, late);
+                v[0] = fma(w.x, a.fx.u, v[0]); v[1] = fma(w.y, a.fx.u, v[1]); v[2] = fma(w.z, a.fx.u, v[2]);
+            }
+            const double3 w = run_list(a.cellsfx, a.cells, kListCap / 2, n, shift, a.fx);
             n = max(n - kListCap / 2, 0);
             v[0] += w.x; v[1] += w.y; v[2] += w.z;
         }
         c = __any_sync(0xffffffffu, open) ? c + 1 : nxt;
         if (steps > guard_max) { overflow = true; break; }
     }
-    const double scale = a.f4pi * a.fx_inv;   // (a power of two: the same rounding)
+    const double scale = a.f4pi * a.fx.inv;   // (a power of two: the same rounding)
     {
-        const double3 w = run_list(a.cellsfx, a.cells, __reduce_max_sync(0xffffffffu, n), n, a.fx_inv);
+        const double3 w = run_list(a.cellsfx, a.cells, __reduce_max_sync(0xffffffffu, n), n, shift, a.fx);
         v[0] = (v[0] + w.x) * scale; v[1] = (v[1] + w.y) * scale; v[2] = (v[2] + w.z) * scale;
     }
     const int late = __reduce_max_sync(0xffffffffu, L.nlate[lane]);
@@ -1815,7 +1832,7 @@ VelArgs make_args(ov_ctx *c, const NodeArrays &na, double t, unsigned long long 
     a.cells = c->tree.cells;
     a.cells32 = c->tree.cells32;
     a.cellsfx = c->tree.cellsfx;
-    a.fx_inv = c->grid_h > 0 ? ov_fx_inv(c) : 0;
+    a.fx = c->fx;
     a.x = na.x; a.y = na.y; a.z = na.z;
     a.tx = na.tx; a.ty = na.ty; a.tz = na.tz;
     a.nx = na.nx; a.ny = na.ny; a.nz = na.nz;
@@ -2792,7 +2809,7 @@ __global__ void __launch_bounds__(kRecThreads, 2) k_rec_far(const __grid_constan
 
 // The segments in fixed point for k_direct_fx: start, vector to the end moved
 // by a period toward it (seg_pwrap), zero where there is none.
-__global__ void k_segments_fx(RecArgs r, double fx_inv, CellFX *__restrict__ out)
+__global__ void k_segments_fx(RecArgs r, FxFrame fx, CellFX *__restrict__ out)
 {
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= r.cap) return;
@@ -2803,16 +2820,17 @@ __global__ void k_segments_fx(RecArgs r, double fx_inv, CellFX *__restrict__ out
         s2[0] = r.x[f]; s2[1] = r.y[f]; s2[2] = r.z[f];
         pwrap_dev(r.geo, s1, s2);
     }
-    bool fits = true;
+    int shift = fx.whole;
     int64_t c[3], s[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        fits = fits && fabs(s1[a] * fx_inv) < kFxLimit && fabs(s2[a] * fx_inv) < kFxLimit;
-        c[a] = __double2ll_rn(s1[a] * fx_inv);
-        s[a] = __double2ll_rn(s2[a] * fx_inv) - c[a];
-        fits = fits && s[a] < (1ll << 61) && s[a] > -(1ll << 61);
+        const double u1 = fma(s1[a], fx.inv, fx.at[a]), u2 = fma(s2[a], fx.inv, fx.at[a]);
+        shift = min(min(shift, fx_shift(u1, s1[a], fx)), fx_shift(u2, s2[a], fx));
+        c[a] = __double2ll_rn(u1);
+        s[a] = __double2ll_rn(u2) - c[a];
+        if (s[a] >= (1ll << 61) || s[a] <= -(1ll << 61)) shift = -1;
     }
-    out[m] = fx_cell(c, s, fits);
+    out[m] = fx_cell(c, s, shift >= 0, shift);
 }
 
 // FP64 direct sums in (node, segment chunk) blocks: each thread takes segments
@@ -2822,13 +2840,13 @@ __global__ void k_segments_fx(RecArgs r, double fx_inv, CellFX *__restrict__ out
 // of the terms' magnitudes.
 // Integer pipe: 16 cycles an interaction and SM.  2,048 nodes of 32,768 with
 // 26 images: 34 ms, 303 with every term in FP64.
-__global__ void __launch_bounds__(kRecThreads, 3) k_direct_fx(RecArgs r, double fx_inv,
+__global__ void __launch_bounds__(kRecThreads, 3) k_direct_fx(RecArgs r, FxFrame fx,
                                                               const CellFX *__restrict__ seg,
                                                               const int *__restrict__ nodes, int n, int span,
                                                               int max_chunks, double *__restrict__ part)
 {
     __shared__ int64_t s_q[OV_MAX_IMAGES + 1][3];
-    __shared__ bool s_in[OV_MAX_IMAGES + 1];
+    __shared__ int s_shift[OV_MAX_IMAGES + 1];   // largest shift of the law (fx_law), -1: out of its range
     __shared__ double red[4][kRecThreads];
     const int b = blockIdx.x, chunk = blockIdx.y;
     if (b >= n) return;
@@ -2848,15 +2866,16 @@ __global__ void __launch_bounds__(kRecThreads, 3) k_direct_fx(RecArgs r, double 
         double q[3];
         if (j < 0) { q[0] = p[0]; q[1] = p[1]; q[2] = p[2]; }
         else image_point(r.geo, j, p, q);
-        bool in = true;
+        int shift = fx.whole;
         for (int a = 0; a < 3; ++a) {
-            in = in && fabs(q[a] * fx_inv) < kFxLimit;
-            s_q[threadIdx.x][a] = __double2ll_rn(q[a] * fx_inv);
+            const double x = fma(q[a], fx.inv, fx.at[a]);
+            shift = min(shift, fx_shift(x, q[a], fx));
+            s_q[threadIdx.x][a] = __double2ll_rn(x);
         }
-        s_in[threadIdx.x] = in;
+        s_shift[threadIdx.x] = shift;
     }
     __syncthreads();
-    const double unit = ldexp(1.0, kFxUnitDirect) * fx_inv * r.f4pi;
+    const double unit = ldexp(1.0, kFxUnitDirect) * fx.inv * r.f4pi;
     double d[3] = {0, 0, 0}, dabs = 0;
     for (int m = m0 + threadIdx.x; m < m1; m += blockDim.x) {
         const int f = r.fwd[m];
@@ -2868,7 +2887,7 @@ __global__ void __launch_bounds__(kRecThreads, 3) k_direct_fx(RecArgs r, double 
         unsigned mask64 = 0;
 #pragma unroll 1
         for (int qi = first; qi < nq; ++qi)
-            if (!fx_law<kFxUnitDirect>(c, s_q[qi], s_in[qi], sum, &mag)) mask64 |= 1u << qi;
+            if (!fx_law<kFxUnitDirect>(c, s_q[qi], s_shift[qi] >= 0, sum, s_shift[qi], &mag)) mask64 |= 1u << qi;
         for (int a = 0; a < 3; ++a) d[a] = fma(fx_value(sum[a]), unit, d[a]);
         dabs = fma((double)mag, unit, dabs);
         for (; mask64 && c.e != kFxZero; mask64 &= mask64 - 1) {
@@ -3210,9 +3229,8 @@ int rec_launch_fx(ov_ctx *c, const RecArgs &ra, const int *d_nodes, int n, int *
         OV_ALLOC(c, cudaMalloc(&c->rec_seg, (size_t)c->cap * sizeof(CellFX)));
         c->rec_seg_cap = c->cap;
     }
-    const double fx_inv = ov_fx_inv(c);
-    k_segments_fx<<<(c->cap + 255) / 256, 256, 0, c->stream>>>(ra, fx_inv, c->rec_seg);
-    k_direct_fx<<<dim3(n, *chunks), kRecThreads, 0, c->stream>>>(ra, fx_inv, c->rec_seg, d_nodes, n, span, *chunks,
+    k_segments_fx<<<(c->cap + 255) / 256, 256, 0, c->stream>>>(ra, c->fx, c->rec_seg);
+    k_direct_fx<<<dim3(n, *chunks), kRecThreads, 0, c->stream>>>(ra, c->fx, c->rec_seg, d_nodes, n, span, *chunks,
                                                                 c->rec_part);
     c->launches += 2;
     return OV_OK;
