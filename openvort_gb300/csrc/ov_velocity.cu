@@ -1901,20 +1901,31 @@ void ov_launch_tangents(ov_ctx *c, const NodeArrays &na, bool lia, cudaStream_t 
 // items for each SM, a walk is split into equal shares of the pre-order cells, so
 // that the launch does not end with a few warps in their last long walk.  Each part
 // pays its item's reads and the way down to its first cell, so not too many.
-// Traversal times (ms) with 1, 2, 4, 8, 16, 32 parts, by items an SM:
-//   496 nodes, 27 query points         3   .202 .150 .121 .098 .125 .190
-//   4,125 nodes, 19                   16  1.061 .778 .520 .399 .405 .481
-//   8,192 nodes, 27                   45   .907 .745 .573 .512 .649
-//   16,384 nodes, 27                  91  1.381 1.202 .953 1.107 1.366
-//   30,009 nodes, walls, 7            43  1.945 1.736 1.423 1.449
-//   32,768 nodes, 27                 182  2.125 1.912 1.925 2.288
-//   49,152 nodes, 27                 273  2.739 2.851 3.034 3.583
-constexpr int kItemsFor8 = 46, kItemsFor4 = 184;
+// Traversal times (ms) with 1, 2, 4, 8, 16, 32 parts, by items an SM and, since
+// walks are longer in larger trees, items times the root of the slots:
+//   496 nodes, 27 query points         3     63   .164 .133 .115 .096 .070 .084
+//   2,048 nodes, 27                   11    515   .322 .272 .240 .184 .170 .244
+//   4,096 nodes, 19                   16   1024   .569 .446 .344 .256 .274 .377
+//   4,096 nodes, 27                   23   1455   .551 .451 .350 .270 .328
+//   24,576 nodes, 7                   35   5545  1.608 1.401 1.145 1.114 1.169
+//   10,240 nodes, 27                  57   5750  1.055 .848 .711 .659 .821
+//   30,009 nodes, walls, 7            43   7490  1.784 1.493 1.444 1.483 1.599
+//   12,288 nodes, 27                  68   7561  1.128 .930 .737 .795
+//   33,536 nodes, 7                   48   8838  1.995 1.733 1.497 1.516
+//   49,152 nodes, 7                   71  15684  2.515 2.214 2.169 2.323
+//   28,672 nodes, 27                 159  26949  1.882 1.714 1.661 1.997
+//   32,768 nodes, 27                 182  32925  2.015 1.880 1.916 2.304
+//   98,304 nodes, 7                  141  44357  4.617 4.590 4.703
+//   40,960 nodes, 27                 227  46015  2.337 2.271 2.427
+//   49,152 nodes, 27                 273  60487  2.701 2.740 2.924
+//   131,072 nodes, walls, 7          189  68290  6.449 6.551 6.715
+// The lines lie about halfway between the rows on either side.
 static int ov_sub_walks(ov_ctx *c, int precision)
 {
     if (!ov_split_walk(c, precision)) return 1;
-    const long long items = (long long)((c->cap + 31) / 32) * ov_query_groups(c) / c->sm_count;
-    return items <= kItemsFor8 ? 8 : (items <= kItemsFor4 ? 4 : 1);
+    const double items = (double)((c->cap + 31) / 32) * ov_query_groups(c) / c->sm_count;
+    const double length = items * sqrt((double)c->cap);
+    return length <= 1000 ? 16 : (length <= 6900 ? 8 : (length <= 27500 ? 4 : (length <= 54000 ? 2 : 1)));
 }
 
 static bool has_mirror_images(const Geometry &g)
@@ -2027,7 +2038,9 @@ static size_t list_bytes(const ov_ctx *c, int precision, int warps)
 }
 
 // Persistent grid: resident blocks per SM (tuned or the occupancy limit) on
-// every SM, but no more blocks than there can be work items.
+// every SM, but no more blocks than there can be work items (a part of a walk is
+// one: 496 nodes 0.096 ms with a warp for each of their 3,888, 0.108 with a warp
+// for every eighth).
 int ov_traversal_blocks(ov_ctx *c, int precision, int warps, int *per_sm)
 {
     VelKernel k = vel_kernel(precision, ov_split_walk(c, precision), warps, mixed_variant(c), has_mirror_images(c->geo));
@@ -2039,7 +2052,8 @@ int ov_traversal_blocks(ov_ctx *c, int precision, int warps, int *per_sm)
     }
     int bps = c->tune.blocks_per_sm > 0 ? std::min(c->tune.blocks_per_sm, occ) : occ;
     if (per_sm) *per_sm = occ;
-    long long items = ((long long)(c->cap + 31) / 32 + (long long)c->mem.size()) * ov_query_groups(c);
+    long long items = ((long long)(c->cap + 31) / 32 + (long long)c->mem.size()) * ov_query_groups(c) *
+                      ov_sub_walks(c, precision);
     long long need = (items + warps - 1) / warps;
     long long blocks = std::min((long long)bps * c->sm_count, need);
     return (int)std::max(1LL, blocks);
