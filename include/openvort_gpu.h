@@ -207,18 +207,18 @@ int ov_set_member_params(ov_ctx *ctx, int i, const ov_params *p);
 /* Launch shape of the traversal: warps per block (2, 4 or 8), query groups
    per node (1-27; 0 = from the node count), persistent blocks per SM (0 =
    the occupancy limit), the order of the work queue (largest member first
-   or member order), and for the mixed traversal the register budget (0:
-   the default; 1: fewer registers for one more resident block).  Results
-   do not depend on it. */
+   or member order), and for the mixed traversal the kernel.  Results do not
+   depend on it. */
 typedef struct ov_tuning {
     int warps_per_block;
     int query_groups;
     int blocks_per_sm;
     int largest_first;
-    int high_occupancy;   /* mixed traversal variant: 0 chosen by the node count, 1 the general
-                             kernel under a tighter register budget; 2, 3, 4 the periodic-image kernel with
-                             fewer values held per lane (mirror images: as 0) with the
-                             compiler's register count, 80 and 64 registers */
+    int high_occupancy;   /* mixed traversal variant: -1 (default) chosen by the (tile, query group)
+                             items an SM; 0 the general kernel, 1 the same under a tighter register
+                             budget; 2, 3, 4 the periodic-image kernel with fewer values held per lane
+                             (mirror images: as 1) with the compiler's register count, 80 and 64
+                             registers */
 } ov_tuning;
 int ov_get_tuning(const ov_ctx *ctx, ov_tuning *out);
 int ov_set_tuning(ov_ctx *ctx, const ov_tuning *tu);

@@ -185,7 +185,7 @@ struct Tuning {
     int groups = 0;        // query groups per node (0: from the node count)
     int blocks_per_sm = 0; // persistent blocks per SM (0: occupancy limit)
     int largest_first = 1; // work queue visits the largest member first
-    int hi_occ = 0;        // mixed traversal: the tighter register budget variant
+    int hi_occ = -1;       // mixed traversal variant (-1: from the work items)
 };
 
 struct ov_ctx {

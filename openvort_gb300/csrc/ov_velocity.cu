@@ -1935,9 +1935,9 @@ static bool has_mirror_images(const Geometry &g)
     return false;
 }
 
-// variant (Tuning::hi_occ) of the mixed traversal: 1 k_vel_mixed under a
-// tighter register budget, 2-4 k_vel_mixp (periodic image sets only) with the
-// compiler's register count, 80 and 64 registers.  0 picks one, all give the
+// variant (Tuning::hi_occ) of the mixed traversal: 0 k_vel_mixed, 1 the same under a
+// tighter register budget, 2-4 k_vel_mixp (periodic image sets only, else as 1) with
+// the compiler's register count, 80 and 64 registers.  -1 picks one, all give the
 // same sums: with at least 48 work items an SM the walk's latency is best hidden by
 // 32 warps (k_vel_mixp at 64 registers, against k_vel_mixed: 262,144 nodes 5.15
 // against 5.5 ms, 1,048,576 20.4 against 24.0); with fewer their tiles lie too far
@@ -1947,7 +1947,8 @@ static bool has_mirror_images(const Geometry &g)
 constexpr int kMixpItems = 48, kFewItems = 40;
 static int mixed_variant(ov_ctx *c)
 {
-    if (c->tune.hi_occ || has_mirror_images(c->geo)) return c->tune.hi_occ;
+    if (c->tune.hi_occ >= 0) return c->tune.hi_occ;
+    if (has_mirror_images(c->geo)) return 0;
     long long tiles = 0;
     for (const Member &m : c->mem) tiles += (m.n + 31) / 32;
     const int G = ov_query_groups(c);

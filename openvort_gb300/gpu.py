@@ -313,7 +313,7 @@ class Context:
         return tu
 
     def set_tuning(self, warps_per_block: int = 4, query_groups: int = 0, blocks_per_sm: int = 0,
-                   largest_first: int = 1, high_occupancy: int = 0):
+                   largest_first: int = 1, high_occupancy: int = -1):
         tu = abi.Tuning(warps_per_block, query_groups, blocks_per_sm, largest_first, high_occupancy)
         self._check(self.lib.ov_set_tuning(self._h, C.byref(tu)))
 
