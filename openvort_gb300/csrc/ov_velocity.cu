@@ -1938,13 +1938,23 @@ static bool has_mirror_images(const Geometry &g)
 // variant (Tuning::hi_occ) of the mixed traversal: 0 k_vel_mixed, 1 the same under a
 // tighter register budget, 2-4 k_vel_mixp (periodic image sets only, else as 1) with
 // the compiler's register count, 80 and 64 registers.  -1 picks one, all give the
-// same sums: with at least 48 work items an SM the walk's latency is best hidden by
-// 32 warps (k_vel_mixp at 64 registers, against k_vel_mixed: 262,144 nodes 5.15
-// against 5.5 ms, 1,048,576 20.4 against 24.0); with fewer their tiles lie too far
-// apart to share cells (32,768 nodes 1.24 against 1.00, 65,536 1.57 against 1.30).
-// Few long items (all 27 query points, or half of them) finish earlier on 24
-// warps than on 20 (114,688 nodes 2.10 against 2.45).  Mirror images: k_vel_mixed.
-constexpr int kMixpItems = 48, kFewItems = 40;
+// same sums.  Traversal times (ms) of variants 0, 1, 4, theta 0.4, 27 query points:
+//   32,768 nodes, 5 groups, 34 items an SM    1.06  1.06  1.31
+//   65,536        3         40                1.24  1.25  1.51
+//   98,304        2         40                1.76  1.78  2.06
+//   114,688       2         47                2.24  1.88  2.17
+//   131,072       2         54                2.48  2.36  2.34
+//   163,840       1         34                3.20  3.19  3.60
+//   212,992       1         44                4.21  3.60  3.98
+//   233,472       1         48                4.39  3.93  4.12
+//   262,144       1         54                4.71  4.56  4.39
+//   1,048,576     1        216               17.77 16.14 15.66
+// (the same order with 7 query points and at theta 0.3, to 2 %).  Many items: the walk's
+// latency is best hidden by 32 warps; with fewer their tiles lie too far apart to
+// share cells.  Few long ones (all query points of a node, or half of them) end
+// earlier on 24 warps than on 20, where the 20 would start a third round.  Mirror
+// images: k_vel_mixed.
+constexpr int kMixpItems = 51, kFewItems = 44;
 static int mixed_variant(ov_ctx *c)
 {
     if (c->tune.hi_occ >= 0) return c->tune.hi_occ;
