@@ -2965,10 +2965,9 @@ struct RecChange {
 // of k_rec_sums, FP64 near the query point.  out: 3 sums, bound.
 __device__ __forceinline__ void corr_point(const RecArgs &r, int k, int j, const RecChange &ch, double out[4])
 {
-    double acc[3] = {0, 0, 0};   // FP64 terms
+    double acc[3] = {0, 0, 0};
     double bound = 0;
-    float tf[3] = {0, 0, 0};     // FP32 terms, their magnitudes' sum sc |R| |s|
-    float mag = 0;
+    float mag = 0;   // of the FP32 terms: sum of sc |R| |s|
     if (k >= 0 && k < r.cap) {
         const double p[3] = {r.x[k], r.y[k], r.z[k]};
         float qg[3], qf[3];
@@ -2980,6 +2979,7 @@ __device__ __forceinline__ void corr_point(const RecArgs &r, int k, int j, const
         for (int i = 0; i < ch.n && i < kRecChangeMax; ++i) {
             int m = ch.m[i], f = ch.f[i];
             if (m < 0 || m >= r.cap || f < 0 || f >= r.cap) continue;
+            if (j < 0 && (m == k || f == k)) continue;   // the node's own segments (where they wrap, too)
             float ag[3], af[3], sv[3];
             bool use64 = false;
             for (int a = 0; a < 3; ++a) {
@@ -3021,17 +3021,16 @@ __device__ __forceinline__ void corr_point(const RecArgs &r, int k, int j, const
             const float sc = __fdividef(r.f4pif * (ra + rb) * ab, fmaf(dot, ab, 1.0f));
             const float slen = sqrtf(fmaf(sv[0], sv[0], fmaf(sv[1], sv[1], sv[2] * sv[2])));
             const float sg = (float)ch.sign[i];   // +-1
-            tf[0] += sg * (fmaf(R[1], sv[2], -R[2] * sv[1]) * sc);
-            tf[1] += sg * (fmaf(R[2], sv[0], -R[0] * sv[2]) * sc);
-            tf[2] += sg * (fmaf(R[0], sv[1], -R[1] * sv[0]) * sc);
+            acc[0] += sg * (fmaf(R[1], sv[2], -R[2] * sv[1]) * sc);
+            acc[1] += sg * (fmaf(R[2], sv[0], -R[0] * sv[2]) * sc);
+            acc[2] += sg * (fmaf(R[0], sv[1], -R[1] * sv[0]) * sc);
             mag += sc * slen * lR2 * ra;
         }
     }
-    // per term 64 eps32 of sc |R| |s| (as k_rec_sums), plus at most 8 eps32 of
-    // the same for the FP32 additions of up to 8 terms; 1.01 covers the
-    // rounding of mag itself
-    for (int a = 0; a < 3; ++a) out[a] = acc[a] + (double)tf[a];
-    out[3] = bound + 1.01 * 72.0 * 5.9604644775390625e-8 * (double)mag;
+    // per term 64 eps32 of sc |R| |s| (as k_rec_sums; they add up in FP64); 1.01
+    // covers the rounding of mag itself
+    for (int a = 0; a < 3; ++a) out[a] = acc[a];
+    out[3] = bound + 1.01 * 64.0 * 5.9604644775390625e-8 * (double)mag;
 }
 
 // Prefetch list of a correction: candidates whose corrections go straight to
