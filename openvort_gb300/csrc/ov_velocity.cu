@@ -2559,6 +2559,10 @@ __global__ void __launch_bounds__(kRecThreads, 3) k_rec_sums(RecArgs r, const in
 // Error of a term relative to sc |R| |s| in units eps32: R 1, |R|^2 3, its
 // inverse root 4.5, the cube 15, the series 5, the sums U 9, the cross product
 // 4: below the 64 that k_rec_finish allows.
+// Measured against FP64, rms per sum of magnitudes over 4,096 candidates (closed form
+// of k_rec_sums in brackets): 65,536 nodes 2.36e-10 (2.52e-10), 10,240 6.2e-10
+// (6.3e-10), 8,250 denser 4.7e-10 (5.0e-10), 16,384 with 7 points 8.0e-10 (7.8e-10);
+// corrections 1.12e-8 (1.21e-8), 1.15e-8 (1.24e-8), 7.9e-9 (8.5e-9), 1.75e-8 (1.94e-8).
 
 // A segment for the series: A = (start's grid part, |s|), B = (midpoint less
 // that, squared distance from which the series holds), C = (s, s^2; 0: no
@@ -2566,6 +2570,7 @@ __global__ void __launch_bounds__(kRecThreads, 3) k_rec_sums(RecArgs r, const in
 struct FarSegment {
     float4 A, B, C;
 };
+constexpr float kFarLengths = 8.0f;
 
 __device__ __forceinline__ FarSegment far_segment(const RecArgs &r, int m, int f)
 {
@@ -2588,7 +2593,7 @@ __device__ __forceinline__ FarSegment far_segment(const RecArgs &r, int m, int f
     }
     const float s2 = fmaf(sv[0], sv[0], fmaf(sv[1], sv[1], sv[2] * sv[2])), slen = sqrtf(s2);
     const float near = sqrtf(r.rnear2) + 0.5f * slen;   // both ends beyond the FP64 radius
-    const float far2 = seg64 ? __int_as_float(0x7f800000) : fmaxf(64.0f * s2, near * near) * 1.0001f;
+    const float far2 = seg64 ? __int_as_float(0x7f800000) : fmaxf(kFarLengths * kFarLengths * s2, near * near) * 1.0001f;
     o.A = make_float4(ag[0], ag[1], ag[2], slen);
     o.B = make_float4(fmaf(0.5f, sv[0], af[0]), fmaf(0.5f, sv[1], af[1]), fmaf(0.5f, sv[2], af[2]), far2);
     o.C = make_float4(sv[0], sv[1], sv[2], seg64 && s2 == 0.0f ? 1e-30f : s2);
@@ -2610,7 +2615,7 @@ __global__ void k_rec_segments(RecArgs r, float4 *__restrict__ seg)
 }
 
 // Segment m -> f at candidate k by the closed form, every query point: t the
-// FP32 sum without kappa / 4 pi, t[3] its magnitude (sc |R| |s|), d the FP64
+// FP32 sum (Kahan) without kappa / 4 pi, t[3] its magnitude (sc |R| |s|), d the FP64
 // sum and its magnitude added.
 __device__ __noinline__ void rec_near(const RecArgs &r, int m, int f, int k, float t[4], double d[4])
 {
@@ -2635,6 +2640,7 @@ __device__ __noinline__ void rec_near(const RecArgs &r, int m, int f, int k, flo
         kg[a] = r.sp[(size_t)a * r.cap + k];
         kf[a] = r.sp[(size_t)(3 + a) * r.cap + k];
     }
+    float c[3] = {0.0f, 0.0f, 0.0f};   // Kahan compensations
     for (int i = 0; i < 4; ++i) t[i] = 0.0f;
     unsigned mask64 = 0;   // query points whose term is done in FP64
 #pragma unroll 3
@@ -2655,9 +2661,9 @@ __device__ __noinline__ void rec_near(const RecArgs &r, int m, int f, int k, flo
         if (use64) mask64 |= 1u << qi;
         if (use64 || nd < 1e-8f) continue;   // (or the ndot filter, far from its threshold)
         const float sc = __fdividef((ra + rb) * ab, fmaf(dot, ab, 1.0f));
-        t[0] = fmaf(fmaf(R[1], sv[2], -R[2] * sv[1]), sc, t[0]);
-        t[1] = fmaf(fmaf(R[2], sv[0], -R[0] * sv[2]), sc, t[1]);
-        t[2] = fmaf(fmaf(R[0], sv[1], -R[1] * sv[0]), sc, t[2]);
+        kahan_add(t[0], c[0], fmaf(R[1], sv[2], -R[2] * sv[1]) * sc);
+        kahan_add(t[1], c[1], fmaf(R[2], sv[0], -R[0] * sv[2]) * sc);
+        kahan_add(t[2], c[2], fmaf(R[0], sv[1], -R[1] * sv[0]) * sc);
         t[3] = fmaf(sc * slen, lR2 * ra, t[3]);
     }
     for (; mask64; mask64 &= mask64 - 1) {
@@ -3056,9 +3062,27 @@ __global__ void k_corr(RecArgs r, const int *__restrict__ cand, int c0, int nc, 
     for (int a = 0; a < 4; ++a) part[(size_t)idx * 4 + a] = out[a];
 }
 
+// An FP32 number as an integer in units of 2^(top - 127 - 23 - 33), top the largest
+// biased exponent of a warp's: exact but for what is below 2^-57 of the largest, and
+// 32 of them add up below 2^62.
+__device__ __forceinline__ int float_exp(float x) { return (int)(__float_as_uint(x) >> 23 & 0xff); }
+__device__ __forceinline__ int64_t float_fixed(float x, int top)
+{
+    const unsigned b = __float_as_uint(x);
+    const int e = (int)(b >> 23 & 0xff), s = e - top + 33;
+    const int m = e ? (int)(b & 0x7fffff | 0x800000) : 0;
+    const int64_t v = s >= 0 ? (int64_t)m << s : (int64_t)(m >> min(-s, 31));
+    return (int)b < 0 ? -v : v;
+}
+// (top 255: some number was infinite or none)
+__device__ __forceinline__ double fixed_value(int64_t v, int top)
+{
+    return top == 255 ? __longlong_as_double(0x7ff8000000000000ll) : (double)v * ldexp(1.0, top - 127 - 23 - 33);
+}
+
 // k_corr and k_corr_finish for image sets that are grids of shifts: a warp takes
 // two candidates and a lane a changed segment, every query point at once by the
-// series of k_rec_far; the lanes' FP32 sums join by shuffles.
+// series of k_rec_far; the lanes' sums join exactly.
 template <int NZ>
 __global__ void __launch_bounds__(256, 2) k_corr_far(const __grid_constant__ RecArgs r, const int *__restrict__ cand,
                                                      int c0, int nc, const __grid_constant__ RecChange ch,
@@ -3090,34 +3114,56 @@ __global__ void __launch_bounds__(256, 2) k_corr_far(const __grid_constant__ Rec
         far_terms<NZ>(R, sv, f2(S.C.w), t, mg, near2);
     }
     const float sg = lane < ch.n ? (float)ch.sign[lane] : 0.0f;   // +-1
-#pragma unroll 1
+    // the lanes join exactly: FP32 sums and magnitudes as integers of one scale, four
+    // values a candidate (FP64 sums as well where some lane was near).  524,288 nodes:
+    // the pairs' decisions 61 ms so, 66 with FP32 sums on all lanes, 76 with FP64 ones.
+    double near64[2][4];
+    int64_t v[8];
+    int top[2][2];
+    bool any_near[2];
+#pragma unroll
     for (int e = 0; e < 2; ++e) {
         float w[4] = {e ? t[0].y : t[0].x, e ? t[1].y : t[1].x, e ? t[2].y : t[2].x, (e ? mg.y : mg.x) * S.A.w};
-        double acc[4] = {0, 0, 0, 0};
+        for (int a = 0; a < 4; ++a) near64[e][a] = 0;
         const bool near = live && !((e ? near2.y : near2.x) >= S.B.w);
-        if (near) rec_near(r, m, f, k[e], w, acc);
-        for (int a = 0; a < 4; ++a) w[a] = live ? (a < 3 ? sg * w[a] : w[a]) : 0.0f;
-        for (int a = 0; a < 3; ++a) acc[a] *= sg;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-            for (int a = 0; a < 4; ++a) w[a] += __shfl_xor_sync(0xffffffffu, w[a], o);
-        if (__any_sync(0xffffffffu, near)) {
+        any_near[e] = __any_sync(0xffffffffu, near);
+        if (any_near[e]) {
+            if (near) rec_near(r, m, f, k[e], w, near64[e]);
+            for (int a = 0; a < 3; ++a) near64[e][a] *= sg;
             for (int o = 16; o > 0; o >>= 1)
-                for (int a = 0; a < 4; ++a) acc[a] += __shfl_xor_sync(0xffffffffu, acc[a], o);
+                for (int a = 0; a < 4; ++a) near64[e][a] += __shfl_xor_sync(0xffffffffu, near64[e][a], o);
         }
-        if (lane != 0 || (e && i1 == i0)) continue;
-        // 64 eps32 a term, 28 for its query points' sum (k_rec_finish), 5 for
-        // the lanes' additions
-        const double eps = 1.01 * 97.0 * 5.9604644775390625e-8;
-        double *cc = corr + 4 * (size_t)(c0 + (e ? i1 : i0));
-        double total = 0;
-        for (int a = 0; a < 3; ++a) {
-            const double d = fma((double)w[a], r.f4pi, acc[a]);
-            cc[a] += d;
-            total += fabs(d);
-        }
-        cc[3] += (eps * r.f4pi * (double)w[3] + 1e-12 * acc[3]) * (1.0 + 1e-9) + 1e-15 * total;
+        for (int a = 0; a < 4; ++a) w[a] = live ? (a < 3 ? sg * w[a] : w[a]) : 0.0f;
+        top[e][0] = __reduce_max_sync(0xffffffffu, max(max(float_exp(w[0]), float_exp(w[1])), float_exp(w[2])));
+        top[e][1] = __reduce_max_sync(0xffffffffu, float_exp(w[3]));
+        for (int a = 0; a < 4; ++a) v[4 * e + a] = float_fixed(w[a], top[e][a == 3]);
     }
+    // each step halves the values a lane keeps: lane 4 i ends with the sum of value i
+#pragma unroll
+    for (int n = 4; n > 0; n >>= 1) {
+        const bool upper = lane & (4 * n);
+#pragma unroll
+        for (int i = 0; i < n; ++i) {
+            const int64_t got = __shfl_xor_sync(0xffffffffu, upper ? v[i] : v[i + n], 4 * n);
+            v[i] = (upper ? v[i + n] : v[i]) + got;
+        }
+    }
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+    const int e = lane >> 4, a = lane >> 2 & 3;
+    const int scale = a == 3 ? (e ? top[1][1] : top[0][1]) : (e ? top[1][0] : top[0][0]);
+    double d = fixed_value(v[0], scale) * r.f4pi;
+    const double n64 = any_near[0] || any_near[1] ? (e ? (a < 2 ? (a ? near64[1][1] : near64[1][0]) : (a == 2 ? near64[1][2] : near64[1][3]))
+                                                       : (a < 2 ? (a ? near64[0][1] : near64[0][0]) : (a == 2 ? near64[0][2] : near64[0][3]))) : 0.0;
+    if (a < 3) d += n64;
+    double total = a < 3 ? fabs(d) : 0.0;
+    total += __shfl_xor_sync(0xffffffffu, total, 4);
+    total += __shfl_xor_sync(0xffffffffu, total, 8);
+    if ((lane & 3) != 0 || (e && i1 == i0)) return;
+    // 64 eps32 a term and 28 for its query points' sum (k_rec_finish); 1.01 covers
+    // the rounding of the magnitudes
+    if (a == 3) d = (1.01 * 92.0 * 5.9604644775390625e-8 * d + 1e-12 * n64) * (1.0 + 1e-9) + 1e-15 * total;
+    corr[4 * (size_t)(c0 + (e ? i1 : i0)) + a] += d;
 }
 
 // The prefetched candidates' corrections into host memory.

@@ -98,3 +98,38 @@ def test_corrections_within_their_bound(images, grid, D, changes):
         if not grid:   # in closed form: 64 eps32 of the terms' magnitudes, which add up in FP64
             assert (step[:, 3] <= 64 * 1.012 * EPS32 * mag + 2e-12 * mag + 1e-14 * np.abs(got[:, :3]).sum(axis=1)).all()
     ctx.close()
+
+
+@pytest.mark.parametrize("images", ["periodic_26", "periodic_6", "open", "wall_2_4"])
+def test_changed_segments_add_up_in_fp64(images):
+    """A segment, another and the first one again with the other sign: what is left is the
+    second one's contribution to FP64 rounding, though the terms are FP32 ones."""
+    begin, correct, fetch, i, d = _functions()
+    base = W.random_walk_tangle(6, 64, D=0.1, seed=9)
+    ht = W.HostTangle(base.pos.copy(), base.conn[:, 0], base.conn[:, 1], base.box_lo, base.box_hi, image_set=images)
+    ctx = gpu.Context(0, params=W.config_params("rw"), precision=abi.OV_PREC_MIXED)
+    ctx.upload(ht)
+    cand = np.arange(0, ht.n, 5, dtype=np.int32)
+    assert begin(ctx.handle, i(cand), len(cand), d(np.zeros((len(cand), 5)))) == 0
+    last = np.zeros((len(cand), 4))
+
+    def added(changes):
+        """The corrections' change by {position in the list: (segment, sign)}; empty positions between."""
+        nonlocal last
+        m, sign = np.full(max(changes) + 1, -1, np.int32), np.zeros(max(changes) + 1)
+        for at, (seg, sg) in changes.items():
+            m[at], sign[at] = seg, sg
+        f = np.where(m >= 0, ht.conn[m, 0], -1).astype(np.int32)
+        assert correct(ctx.handle, 0, len(cand), i(m), i(f), d(sign), len(m), i(cand), 0) == 0
+        got = np.zeros((len(cand), 4))
+        assert fetch(ctx.handle, 0, len(cand), d(got)) == 0
+        step, last = got - last, got
+        return step[:, :3]
+
+    for one, two in ((3, 200), (130, 77), (301, 9)):
+        first, second = added({0: (one, 1.0)}), added({0: (two, 1.0)})
+        both = added({0: (one, 1.0), 16: (two, 1.0), 1: (one, -1.0)})
+        # three additions of the terms, and those of the running sums
+        scale = np.abs(first) + np.abs(second) + np.abs(last[:, :3])
+        assert (np.abs(both - second) <= 16 * 2.0 ** -53 * scale).all()
+    ctx.close()
