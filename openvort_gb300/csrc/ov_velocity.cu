@@ -3160,9 +3160,9 @@ __global__ void __launch_bounds__(256, 2) k_corr_far(const __grid_constant__ Rec
     total += __shfl_xor_sync(0xffffffffu, total, 4);
     total += __shfl_xor_sync(0xffffffffu, total, 8);
     if ((lane & 3) != 0 || (e && i1 == i0)) return;
-    // 64 eps32 a term and 28 for its query points' sum (k_rec_finish); 1.01 covers
-    // the rounding of the magnitudes
-    if (a == 3) d = (1.01 * 92.0 * 5.9604644775390625e-8 * d + 1e-12 * n64) * (1.0 + 1e-9) + 1e-15 * total;
+    // 64 eps32 a term (the series' 42 have its query points' sum in them) and 2 for the
+    // near ones' Kahan sum; 1.01 covers the rounding of the magnitudes
+    if (a == 3) d = (1.01 * 66.0 * 5.9604644775390625e-8 * d + 1e-12 * n64) * (1.0 + 1e-9) + 1e-15 * total;
     corr[4 * (size_t)(c0 + (e ? i1 : i0)) + a] += d;
 }
 
