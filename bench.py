@@ -35,9 +35,9 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 METRIC = "biot_savart_node_evals_per_s"
-# DRAM bytes (read + write) of one FP64 traversal launch on this workload, from an ncu capture
-# (dram__bytes_read.sum + dram__bytes_write.sum of k_vel_fp64, two launches: 9.87 and 9.92 MB)
-K_VEL_FP64_DRAM_BYTES = 23.604e6   # k_vel_split: 20.34 MB read + 3.26 MB written (ncu)
+# DRAM bytes of one FP64 traversal launch on this workload, from an ncu capture of k_vel_split
+# (dram__bytes_read.sum + dram__bytes_write.sum: 20.36 + 3.25 MB)
+K_VEL_FP64_DRAM_BYTES = 23.611e6
 UNIT = "node-evals/s"
 WORKLOAD = dict(workload="random-walk tangle, 256 loops x 256 nodes (65,536), D=0.1 cm, periodic_26, "
                          "theta=0.4, one update_tangle per step",
@@ -673,8 +673,9 @@ def run_ours(args):
     value = world * n / (mean_ms * 1e-3)
     phases = np.mean(np.array(trav_ms), axis=0).tolist()
 
-    # ---- roofline of the dominant kernel: the FP64 traversal, against the FP64 FMA peak.  Its
-    # interactions run on 64-bit integer mantissas, so it may pass that peak; the integer pipe bounds it
+    # ---- roofline of the dominant kernel, the FP64 traversal: its interactions run on 64-bit integer
+    # mantissas, so its peak is the rate of that law with every lane busy (the direct sums, timed
+    # below); the FP64 FMA peak is of a pipe that it leaves nearly idle
     acc, vis = st["accepts"], st["visits"]
     flops = 42 * acc + 9 * vis   # algorithmic flops per launch (fixed convention, whatever pipe runs them)
     trav_s = phases[2] * 1e-3
@@ -812,7 +813,10 @@ def run_ours(args):
     ctx.upload(ht)
     ctx.update_tangle(0.0)
     sub = direct_subsample(n, 4096, 1)
+    ctx.direct_velocities(sub)   # (allocates)
+    ctx.timer_start()
     direct_v, _ = ctx.direct_velocities(sub)
+    law_rate = len(sub) * n * (1 + ht.n_images) / (ctx.timer_stop() * 1e-3)   # interactions/s
     fp64_vs_direct = rel_l2(fp64_vels[sub], direct_v)
     if isinstance(mixed, dict) and "value" in mixed:
         mixed["rel_l2_vs_direct_subsample"] = rel_l2(mixed_vels[sub], direct_v)
@@ -864,14 +868,17 @@ def run_ours(args):
         "l2": "flushed between timed steps (256 MiB write)",
         "parallelism": "replicas" if world > 1 else "single GPU",
         "phases_ms": {"tangents": phases[0], "tree_build": phases[1], "traversal": phases[2]},
-        "roofline": {"bound": "integer issue", "pipe": "fp64", "achieved": achieved, "peak": fp64_peak,
-                     "unit": "TFLOP/s", "frac": achieved / fp64_peak, "traffic": K_VEL_FP64_DRAM_BYTES,
+        "roofline": {"bound": "integer pipe", "pipe": "integer", "achieved": acc / trav_s / 1e9,
+                     "peak": law_rate / 1e9, "unit": "G interactions/s", "frac": acc / trav_s / law_rate,
+                     "traffic": K_VEL_FP64_DRAM_BYTES,
                      "traffic_note": "DRAM bytes per launch from ncu; the traversal is bound by the integer pipe",
-                     "peak_source": "measured in this run (FP64 FMA chains, all SMs)",
-                     "work": "42 flops per accepted interaction + 9 per visited cell (fixed convention); the split "
-                             "walk runs the visits' tests in FP32 and the interactions on 64-bit integer "
-                             "mantissas, so the fraction is of a peak whose pipe it leaves nearly idle",
-                     "accepts": acc, "visits": vis, "fp32_fma_peak_tflops": fp32_peak,
+                     "peak_source": "measured in this run: the same law with every lane busy and no walk (FP64 direct "
+                                    "sums of 4,096 nodes over all segments and query points)",
+                     "work": "accepted interactions (the walk's visits count as none)",
+                     "tflops_convention": achieved,
+                     "tflops_note": "42 flops per accepted interaction + 9 per visited cell, whatever pipe runs them",
+                     "accepts": acc, "visits": vis, "fp64_fma_peak_tflops": fp64_peak,
+                     "fp32_fma_peak_tflops": fp32_peak,
                      "warp_efficiency": vis / max(1, 32 * st["warp_steps"])},
         "accuracy": {"fp64_tree_rel_l2_vs_direct_subsample": fp64_vs_direct,
                      "subsample": "4,096 nodes, FP64 direct sums (tree == NULL branch) on the GPU"},
