@@ -175,7 +175,8 @@ static void release_buffers(ov_ctx *c)
     c->fwd = c->rev = c->status = c->pin = c->dnodes = c->d_tid = c->d_qorder = nullptr;
     c->d_tprm = nullptr;
     c->d_mrange = nullptr;
-    c->d_pairs = c->d_npairs = c->d_loop_off = c->d_loop_nodes = nullptr;
+    c->d_pairs = c->d_loop_off = c->d_loop_nodes = nullptr;
+    c->d_npairs = nullptr;
     c->d_loop_buf = c->d_loop_cut = nullptr;
     c->rec_nodes = c->rec_pair = nullptr;
     c->rec_out = c->rec_corr = c->rec_part = nullptr;

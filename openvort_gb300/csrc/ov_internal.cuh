@@ -236,7 +236,8 @@ struct ov_ctx {
     // reconnect / smoothing scratch
     uint64_t *d_gkeys = nullptr, *d_gkeys_alt = nullptr;
     int *d_gidx = nullptr, *d_gidx_alt = nullptr;
-    int *d_pairs = nullptr, *d_npairs = nullptr;
+    int *d_pairs = nullptr;
+    unsigned long long *d_npairs = nullptr;
     int pair_cap = 0;
     int *d_loop_nodes = nullptr, *d_loop_off = nullptr;
     double *d_loop_buf = nullptr;

@@ -387,7 +387,8 @@ __device__ __forceinline__ bool clearly_apart(const Geometry &geo, const double 
 __global__ void k_pairs(const uint64_t *__restrict__ keys, const int *__restrict__ idx, int cap,
                         const double *__restrict__ x, const double *__restrict__ y, const double *__restrict__ z,
                         GridGeom gg, Geometry geo, double rec_dist, const int *__restrict__ tid,
-                        const DevParams *__restrict__ tprm, int *__restrict__ pairs, int *npairs, int pair_cap)
+                        const DevParams *__restrict__ tprm, int *__restrict__ pairs, unsigned long long *npairs,
+                        int pair_cap)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= cap) return;
@@ -433,8 +434,9 @@ __global__ void k_pairs(const uint64_t *__restrict__ keys, const int *__restrict
                     pwrap_dev(geo, pk, v2);
                     double d = len3_ref(rn_sub(pk[0], v2[0]), rn_sub(pk[1], v2[1]), rn_sub(pk[2], v2[2]));
                     if (d > rec_dist) continue;
-                    int slot = atomicAdd(npairs, 1);
-                    if (slot < pair_cap) { pairs[2 * slot] = k; pairs[2 * slot + 1] = l; }
+                    // (nodes crowded within rec_dist make more pairs than an int counts)
+                    const unsigned long long slot = atomicAdd(npairs, 1ull);
+                    if (slot < (unsigned long long)pair_cap) { pairs[2 * slot] = k; pairs[2 * slot + 1] = l; }
                 }
             }
         }
@@ -1291,13 +1293,15 @@ int hremesh(ov_ctx *c, int mi, double min_dist, double max_dist, double time, in
     return OV_OK;
 }
 
+constexpr long long kMaxPairs = 1ll << 30;   // 8 GB of pairs
+
 int ensure_pairs(ov_ctx *c, int need)
 {
     if (c->pair_cap >= need && c->d_pairs) return OV_OK;
     if (c->d_pairs) cudaFree(c->d_pairs);
     c->d_pairs = nullptr;
     OV_ALLOC(c, cudaMalloc(&c->d_pairs, (size_t)need * 2 * sizeof(int)));
-    if (!c->d_npairs) OV_ALLOC(c, cudaMalloc(&c->d_npairs, sizeof(int)));
+    if (!c->d_npairs) OV_ALLOC(c, cudaMalloc(&c->d_npairs, sizeof *c->d_npairs));
     c->pair_cap = need;
     return OV_OK;
 }
@@ -1317,7 +1321,7 @@ int find_pairs(ov_ctx *c, std::vector<std::pair<int, int>> &out)
         gg.n[a] = (int)std::max(1.0, std::min(cells, 1024.0));
         gg.periodic[a] = c->geo.periodic[a];
     }
-    int r = ensure_pairs(c, std::max(c->pair_cap, 4 * std::max(c->n_live, 16)));
+    int r = ensure_pairs(c, std::max(c->pair_cap, (int)std::min(4ll * std::max(c->n_live, 16), kMaxPairs)));
     if (r) return r;
     TreeBuf &t = c->tree;
     int nb = (cap + 255) / 256;
@@ -1326,18 +1330,21 @@ int find_pairs(ov_ctx *c, std::vector<std::pair<int, int>> &out)
     c->launches++;
     ov_sort_keys(c, t, cap, c->stream);
     for (int attempt = 0; attempt < 2; ++attempt) {
-        OV_CUDA(c, cudaMemsetAsync(c->d_npairs, 0, sizeof(int), c->stream));
+        OV_CUDA(c, cudaMemsetAsync(c->d_npairs, 0, sizeof *c->d_npairs, c->stream));
         const bool ens = c->mem.size() > 1;
         k_pairs<<<nb, 256, 0, c->stream>>>(t.keys, t.order, cap, c->node.x, c->node.y, c->node.z, gg, c->geo, rd,
                                            ens ? c->d_tid : nullptr, ens ? c->d_tprm : nullptr, c->d_pairs,
                                            c->d_npairs, c->pair_cap);
         c->launches++;
         OV_CUDA(c, cudaGetLastError());
-        int np = 0;
-        OV_CUDA(c, cudaMemcpyAsync(&np, c->d_npairs, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+        unsigned long long found = 0;
+        OV_CUDA(c, cudaMemcpyAsync(&found, c->d_npairs, sizeof found, cudaMemcpyDeviceToHost, c->stream));
         OV_CUDA(c, cudaStreamSynchronize(c->stream));
+        if (found > (unsigned long long)kMaxPairs)
+            return ov_fail(c, OV_ERR_ARG, "reconnect: %llu pairs of nodes within rec_dist", found);
+        const int np = (int)found;
         if (np > c->pair_cap) {
-            if ((r = ensure_pairs(c, np + np / 2))) return r;
+            if ((r = ensure_pairs(c, (int)std::min(np + np / 2ll, kMaxPairs)))) return r;
             continue;
         }
         std::vector<int> buf(2 * (size_t)np);
