@@ -209,13 +209,15 @@ FX_INLINE int64_t fx_sqrt(int64_t a)
     const float f = fmaf((float)(unsigned)fx_hi(a), 4294967296.0f, (float)(unsigned)a);
     const float y = fx_rsqrt(f);
     const int m = fx_int(f * y);
-    // a = (m + w / 2^16 + v / 2^32)^2: w and v from exact residuals.  (w^2 is taken by
-    // itself: a factor m + w / 2^17 rounded to 32 bits costs the second residual w / 2,
-    // 2^-49 of the root at the lower end; it saves 0.7 % of an evaluation.)
+    // a = (m + w / 2^16 + v / 2^32)^2: w from an exact residual, v from what that leaves
+    // less w^2, whose FP32 value does.  (A factor m + w / 2^17 rounded to 32 bits costs
+    // the second residual w / 2, 2^-49 of the root at the lower end; w^2 in integers
+    // 0.5 to 1 % of an evaluation.)
     const int64_t r = fx_mad(-m, m, a);
-    const int w = fx_int((float)(int)(r >> 10) * (y * 33554432.0f));
+    const float wf = (float)(int)(r >> 10) * (y * 33554432.0f);
+    const int w = fx_int(wf);
     const int64_t r2 = fx_mad(-w, m, r << 15);
-    const int v = fx_int((float)((int)(r2 >> 4) - (int)(fx_mul(w, w) >> 21)) * (y * 1048576.0f));
+    const int v = fx_int(fmaf(wf * -4.76837158203125e-7f, wf, (float)(int)(r2 >> 4)) * (y * 1048576.0f));
     return fx_mad(w, 65536, v) + ((int64_t)m << 32);
 }
 

@@ -2870,7 +2870,7 @@ __global__ void k_segments_fx(RecArgs r, FxFrame fx, CellFX *__restrict__ out)
 // after the loop.  Layout of part as k_rec_sums: the sums, then in [4] the sum
 // of the terms' magnitudes.
 // Integer pipe: 16 cycles an interaction and SM.  2,048 nodes of 32,768 with
-// 26 images: 34 ms, 303 with every term in FP64.
+// 26 images: 25.9 ms, 303 with every term in FP64.
 __global__ void __launch_bounds__(kRecThreads, 3) k_direct_fx(RecArgs r, FxFrame fx,
                                                               const CellFX *__restrict__ seg,
                                                               const int *__restrict__ nodes, int n, int span,
@@ -3992,7 +3992,7 @@ __global__ void k_sph_points(SphArgs s)
 // cells evaluated by the integer law.  Persistent warps take (query point, part,
 // tile) items: the walks differ in length, and with one warp of a fixed grid for
 // each the SMs were busy for 4.2 to 14.8 million cycles (16,000 nodes,
-// 7.15 ms; an evaluation 8.1 ms, 4.4 now).
+// 7.15 ms; an evaluation 8.1 ms, 4.5 now).
 __global__ void __launch_bounds__(128, 4) k_sph_query_split(SphArgs s, double *__restrict__ part)
 {
     const VelArgs &a = s.v;
